@@ -5,7 +5,8 @@ Kernel sources are plain CUDA (no torch headers) compiled by nvcc with
 cross-compiles without a GPU, so this runs on the CPU build box; the resulting ``.so`` travels to the
 GPU box with the repo snapshot (it is git-ignored).
 
-``python -m mlx_sharding_b200.ops.build [--force] [--verbose]``
+``python -m mlx_sharding_b200.ops.build [--force] [--verbose]``; ``python mlx_sharding_b200/ops/build.py --gemm-sources`` prints the paths
+of the bf16 GEMM's sources.
 """
 from __future__ import annotations
 
@@ -22,7 +23,9 @@ OBJ = os.path.join(HERE, "_build")
 MODULE = "_b200_C"
 SO_PATH = os.path.join(HERE, MODULE + ".so")
 
-CU_SOURCES = ["gemm_tcgen05.cu", "gemm_persistent.cu", "gemm_pair.cu", "gemm_q_tcgen05.cu", "gemm_q_persistent.cu", "gemm_fp8.cu", "elementwise.cu", "attention.cu", "attention_prefill.cu", "flash_tc.cu", "mla_decode.cu", "moe.cu", "sampler.cu", "p2p.cu", "ep.cu", "hybrid.cu", "diffattn.cu", "streams.cu", "sinkattn.cu", "selscan.cu", "headdelta.cu"]
+# the bf16 GEMM: what the stand-alone harness (tests/cuda/build.sh) links, too
+GEMM_SOURCES = ["gemm_tcgen05.cu", "gemm_persistent.cu", "gemm_pair.cu"]
+CU_SOURCES = GEMM_SOURCES + ["gemm_q_tcgen05.cu", "gemm_q_persistent.cu", "gemm_fp8.cu", "elementwise.cu", "attention.cu", "attention_prefill.cu", "flash_tc.cu", "mla_decode.cu", "moe.cu", "sampler.cu", "p2p.cu", "ep.cu", "hybrid.cu", "diffattn.cu", "streams.cu", "sinkattn.cu", "selscan.cu", "headdelta.cu"]
 # exact-mode kernels (fp32 recurrences, rotary angles of long positions): IEEE division / exp / sincos
 NO_FAST_MATH = {"hybrid.cu", "diffattn.cu", "streams.cu", "sinkattn.cu", "selscan.cu", "headdelta.cu"}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -102,5 +105,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 if __name__ == "__main__":
+    if "--gemm-sources" in sys.argv:
+        print("\n".join(os.path.join(CSRC, f) for f in GEMM_SOURCES))
+        sys.exit(0)
     p = build(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     print(p)

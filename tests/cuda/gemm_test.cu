@@ -160,6 +160,11 @@ int main(int argc, char** argv) {
   { Case c; c.name = "grouped"; c.m = 48; c.n = 256; c.k = 512; c.E = 8; cases.push_back(c); }
   { Case c; c.name = "grouped_dual"; c.m = 96; c.n = 384; c.k = 512; c.E = 16; c.dual = true; cases.push_back(c); }
   { Case c; c.name = "grouped_big_rows"; c.m = 2000; c.n = 256; c.k = 256; c.E = 4; cases.push_back(c); }
+  // more than 256 rows: tiles on pairs of SMs (gemm_pair.cu), every epilogue, a last tile of one row
+  { Case c; c.name = "pair_res_bias_m513"; c.m = 513; c.n = 392; c.k = 200; c.res = true; c.bias = true; cases.push_back(c); }
+  { Case c; c.name = "pair_dual_m300"; c.m = 300; c.n = 264; c.k = 512; c.dual = true; cases.push_back(c); }
+  { Case c; c.name = "pair_fp32_m257"; c.m = 257; c.n = 1000; c.k = 136; c.fp32 = true; cases.push_back(c); }
+  { Case c; c.name = "pair_grouped_dual"; c.m = 3000; c.n = 384; c.k = 320; c.E = 9; c.dual = true; c.bn = 256; cases.push_back(c); }
   if (!quick) {
     // model shapes (DeepSeek-V2-Lite / Llama-3-8B), with timing
     { Case c; c.name = "dsv2_qkv_a_m64"; c.m = 64; c.n = 3648; c.k = 2048; c.iters = 20; cases.push_back(c); }
