@@ -479,7 +479,7 @@ bool flash_prefill_takes(const Tensor& q, const Tensor& kpool, const Tensor& vpo
 }
 
 Tensor flash_prefill(const Tensor& q, const Tensor& kpool, const Tensor& vpool, const Tensor& block_tables, const Tensor& cu_seqlens,
-                     const Tensor& context_lens, double scale, int64_t num_tokens, double softcap, int64_t max_ctx) {
+                     const Tensor& context_lens, double scale, int64_t num_tokens, double softcap, int64_t max_ctx, int64_t wait_spins) {
   check_bf16(q, "q"); check_bf16(kpool, "kpool"); check_bf16(vpool, "vpool");
   TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && kpool.is_contiguous() && vpool.is_contiguous());
   TORCH_CHECK(block_tables.scalar_type() == torch::kInt32 && block_tables.is_contiguous() && cu_seqlens.scalar_type() == torch::kInt32 &&
@@ -491,7 +491,7 @@ Tensor flash_prefill(const Tensor& q, const Tensor& kpool, const Tensor& vpool, 
   a.block_tables = block_tables.data_ptr<int>(); a.max_blocks = (int)block_tables.size(1);
   a.cu_seqlens = cu_seqlens.data_ptr<int>(); a.context_lens = context_lens.data_ptr<int>();
   a.num_seqs = (int)context_lens.numel(); a.max_tiles = (int)((num_tokens + 63) / 64 + a.num_seqs);
-  a.scale = (float)scale; a.out = out.data_ptr();
+  a.scale = (float)scale; a.out = out.data_ptr(); a.wait_spins = (uint32_t)wait_spins;
   const bool mma_sync = softcap == 0.0 && b200::flash_prefill_supported(a.dk_, a.dv_);
   if (b200::flash_tc_supported(a) && !(mma_sync && flash_short(max_ctx, num_tokens, a.num_seqs, a.q_heads))) {
     LAUNCH_OK(b200::flash_tc_launch(a, cur_stream()));
@@ -1634,7 +1634,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mla_rope_kv_write", &mla_rope_kv_write);
   m.def("paged_attention", &paged_attention);
   m.def("flash_prefill", &flash_prefill, py::arg("q"), py::arg("kpool"), py::arg("vpool"), py::arg("block_tables"), py::arg("cu_seqlens"),
-        py::arg("context_lens"), py::arg("scale"), py::arg("num_tokens"), py::arg("softcap") = 0.0, py::arg("max_ctx") = 0);
+        py::arg("context_lens"), py::arg("scale"), py::arg("num_tokens"), py::arg("softcap") = 0.0, py::arg("max_ctx") = 0,
+        py::arg("wait_spins") = (int64_t)b200::kWaitSpins);
   m.def("flash_prefill_takes", &flash_prefill_takes);
   m.def("mla_prefill_prologue", &mla_prefill_prologue);
   m.def("flash_mla", &flash_mla);

@@ -64,6 +64,7 @@ struct FlashTcParams {
   const float* sink; const __nv_bfloat16* gate; long long ld_gate;
   int gate_elem, block, window, keep;
   float out_mult;
+  uint32_t wait_spins = kWaitSpins;            // bound of every wait
 };
 
 __host__ __device__ constexpr int ft_streams(int dv) { return dv > 128 ? 1 : 2; }
@@ -260,11 +261,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_smem;
   const int total = s_cum[p.num_seqs - 1], items = total * heads;
-  // the i-th item of this CTA, as the producer drew and laid it out; false at the end of the list
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(bar, parity, dead, p.wait_spins); };
+  // the i-th item of this CTA, as the producer drew and laid it out; false at the end of the list, or where a wait gave up
   auto item_at = [&](uint32_t i, FlashItem& it) {
-    mbar_wait_bounded(&w_full[i % kSlots], (i / kSlots) & 1, dead);
+    const bool here = wait(&w_full[i % kSlots], (i / kSlots) & 1);
     it = s_item[i % kSlots];
-    return it.n_max >= 0 && *reinterpret_cast<volatile uint32_t*>(dead) == 0u;
+    return here && it.n_max >= 0 && *reinterpret_cast<volatile uint32_t*>(dead) == 0u;
   };
 
   if (warp == 8) {
@@ -274,16 +276,17 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
       for (int s = 0; s < NS; ++s) qn[s] = 0;
       int w = blockIdx.x;
-      for (uint32_t i = 0;; ++i) {
+      bool alive = true;                                                        // a copy is armed only on a barrier whose last one has been waited for
+      for (uint32_t i = 0; alive; ++i) {
         if (i > 0) {                                                            // the item of a CTA that was taken out of the launch queue
-          mbar_wait_bounded(clc_bar, (i - 1) & 1, dead);
+          if (!wait(clc_bar, (i - 1) & 1)) break;
           w = ft_canceled_cta(s_clc, items);
         }
-        const bool more = w < items && *reinterpret_cast<volatile uint32_t*>(dead) == 0u;
+        const bool more = w < items;
         FlashItem it = {};
         it.n_max = -1;
         if (more) it = ft_item<NS, MODE>(p, s_cum, s_start, s_ctx, w, total, heads, pair_heads);
-        mbar_wait_bounded(&w_empty[i % kSlots], ((i / kSlots) & 1) ^ 1, dead);
+        if (!wait(&w_empty[i % kSlots], ((i / kSlots) & 1) ^ 1)) break;
         s_item[i % kSlots] = it;
         mbar_arrive(&w_full[i % kSlots]);
         if (!more) break;
@@ -309,26 +312,29 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
           for (int s = 0; s < NS; ++s) {
             if (it.n[s] == 0) continue;
-            mbar_wait_bounded(&q_empty[s], (qn[s] & 1) ^ 1, dead);
+            alive = alive && wait(&q_empty[s], (qn[s] & 1) ^ 1);
+            if (!alive) continue;
             mbar_arrive_expect_tx(&q_full[s], QB);
             for (int c = 0; c < CK; ++c) ft_tma_3d(smem_u32(q_smem + s * QB + c * kRows * 128), &tmap_q, &q_full[s], c * 64, it.head[s], it.tok[s]);
             ++qn[s];
           }
         }
-        for (int j = 0; j < it.n_max; ++j, ++kv) {
+        for (int j = 0; alive && j < it.n_max; ++j, ++kv) {
           const int st = kv % ST;
           const uint32_t ph = (kv / ST) & 1;
           const int key0 = it.tile(j) * kKeys, nbox = min(per, (kv_end - key0 + R - 1) / R);
           const uint32_t kd = smem_u32(k_smem + st * KB), vd = smem_u32(v_smem + st * VB);
           int ahead[4] = {0, 0, 0, 0};
           if (j + 1 < it.n_max) rows_of(j + 1, ahead);
-          mbar_wait_bounded(&k_empty[st], ph ^ 1, dead);
+          alive = wait(&k_empty[st], ph ^ 1);
+          if (!alive) break;
           if constexpr (MLA) {
             const int lin = (int)(lin0 + key0);
             mbar_arrive_expect_tx(&k_full[st], KB);
             for (int c = 0; c < CK - 1; ++c) ft_tma_2d(kd + c * CHUNK, &tmap_k, &k_full[st], it.head[0] * (DK - 64 + DV) + c * 64, lin);
             ft_tma_2d(kd + (CK - 1) * CHUNK, &tmap_pe, &k_full[st], 512, row[0]);
-            mbar_wait_bounded(&v_empty[st], ph ^ 1, dead);
+            alive = wait(&v_empty[st], ph ^ 1);
+            if (!alive) break;
             mbar_arrive_expect_tx(&v_full[st], VB);
             for (int c = 0; c < CV; ++c) ft_tma_2d(vd + c * CHUNK, &tmap_k, &v_full[st], it.head[0] * (DK - 64 + DV) + DK - 64 + c * 64, lin);
           } else {
@@ -337,7 +343,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             for (int b = 0; b < 4; ++b)
               if (b < nbox)
                 for (int c = 0; c < CK; ++c) ft_tma_2d(kd + c * CHUNK + b * R * 128, &tmap_k, &k_full[st], c * 64, row[b]);
-            mbar_wait_bounded(&v_empty[st], ph ^ 1, dead);
+            alive = wait(&v_empty[st], ph ^ 1);
+            if (!alive) break;
             mbar_arrive_expect_tx(&v_full[st], nbox * R * DV * 2);
 #pragma unroll
             for (int b = 0; b < 4; ++b)
@@ -357,17 +364,20 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       uint32_t kv = 0, g = 0, cnt = 0;                                          // key tiles of the CTA, tiles and items of the stream so far
       const uint32_t qa = smem_u32(q_smem + s * QB);
       FlashItem it;
-      for (uint32_t i = 0; item_at(i, it); ++i) {
+      bool alive = true;
+      for (uint32_t i = 0; alive && item_at(i, it); ++i) {
         mbar_arrive(&w_empty[i % kSlots]);
         const int n = s ? it.n[1] : it.n[0];
-        if (n > 0) mbar_wait_bounded(&q_full[s], cnt & 1, dead);
-        for (int j = 0; j < it.n_max; ++j, ++kv) {
-          mbar_wait_bounded(&k_full[kv % ST], (kv / ST) & 1, dead);
+        if (n > 0) alive = wait(&q_full[s], cnt & 1);
+        for (int j = 0; alive && j < it.n_max; ++j, ++kv) {
+          alive = wait(&k_full[kv % ST], (kv / ST) & 1);
+          if (!alive) break;
           if (j >= n) {                                                         // (rows in pairs: the first tile sees fewer keys)
             mbar_arrive(&k_empty[kv % ST]);
             continue;
           }
-          if (g >= NB) mbar_wait_bounded(&o_done[s * NB + g % NB], (g / NB - 1) & 1, dead);       // the product that read this buffer's P
+          if (g >= NB) alive = wait(&o_done[s * NB + g % NB], (g / NB - 1) & 1);                   // the product that read this buffer's P
+          if (!alive) break;
           tc_fence_after();
           const uint32_t ka = smem_u32(k_smem + (kv % ST) * KB), d = tmem_base + (s * NB + g % NB) * 64;
 #pragma unroll
@@ -394,15 +404,17 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (elect_one()) {
       uint32_t kv = 0, g[2] = {0, 0}, cnt[2] = {0, 0};
       FlashItem it;
-      for (uint32_t i = 0; item_at(i, it); ++i) {
+      bool alive = true;
+      for (uint32_t i = 0; alive && item_at(i, it); ++i) {
         mbar_arrive(&w_empty[i % kSlots]);
-        for (int j = 0; j < it.n_max; ++j, ++kv) {
-          mbar_wait_bounded(&v_full[kv % ST], (kv / ST) & 1, dead);
+        for (int j = 0; alive && j < it.n_max; ++j, ++kv) {
+          alive = wait(&v_full[kv % ST], (kv / ST) & 1);
 #pragma unroll
           for (int s = 0; s < NS; ++s) {
             if (j >= it.n[s]) continue;
-            if (j == 0 && cnt[s] > 0) mbar_wait_bounded(&o_free[s], (cnt[s] - 1) & 1, dead);      // the last item's result has been read
-            mbar_wait_bounded(&p_ready[s * NB + g[s] % NB], (g[s] / NB) & 1, dead);
+            if (j == 0 && cnt[s] > 0) alive = alive && wait(&o_free[s], (cnt[s] - 1) & 1);        // the last item's result has been read
+            alive = alive && wait(&p_ready[s * NB + g[s] % NB], (g[s] / NB) & 1);
+            if (!alive) continue;
             tc_fence_after();
             const uint32_t va = smem_u32(v_smem + (kv % ST) * VB), pa = tmem_base + (s * NB + g[s] % NB) * 64, d = tmem_base + O_COL + s * DV;
 #pragma unroll
@@ -434,8 +446,16 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     constexpr int OCOLS = NS == 2 ? DV : DV / 2;                                 // accumulator columns that this thread rescales and stores
     uint32_t g = 0, kv0 = 0, cnt = 0;                                            // tiles of the stream, key tiles of the CTA, items of the stream so far
     FlashItem it;
-    for (uint32_t i = 0; item_at(i, it); ++i) {
+    for (uint32_t i = 0;; ++i) {
+      // threads that meet at a barrier, a shuffle or a warp-wide access to TMEM below leave at the same item.  (Where a wait gives up inside an
+      // item its later ones fall through, and the item is walked to its end.)
+      const bool on = item_at(i, it);
       __syncwarp();
+      if constexpr (NS == 1) {
+        if (!named_bar_and(3, 256, on)) break;
+      } else {
+        if (!__all_sync(0xffffffffu, on)) break;
+      }
       if (lane == 0) mbar_arrive(&w_empty[i % kSlots]);
       const int n = s ? it.n[1] : it.n[0], pos0 = s ? it.pos[1] : it.pos[0], rows = s ? it.rows[1] : it.rows[0], kv_end = s ? it.end[1] : it.end[0];
       const int tok = s ? it.tok[1] : it.tok[0], head = s ? it.head[1] : it.head[0];
@@ -446,7 +466,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if constexpr (SINK) {
         // this row's query as two bf16 terms, in the K-major 128B-swizzled layout that TMA writes
-        mbar_wait_bounded(&q_empty[s], (cnt & 1) ^ 1, dead);
+        wait(&q_empty[s], (cnt & 1) ^ 1);
         constexpr int LPR = DK / 4, RPI = 32 / LPR;                              // lanes of a row, rows of an instruction: whole rows, coalesced
         const int c4 = lane % LPR;
 #pragma unroll 8
@@ -468,7 +488,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
       for (int j = 0; j < n; ++j, ++g) {
         const uint32_t buf = tmem_base + lane_addr + (s * NB + g % NB) * 64;
-        mbar_wait_bounded(&s_full[s * NB + g % NB], (g / NB) & 1, dead);
+        wait(&s_full[s * NB + g % NB], (g / NB) & 1);
         tc_fence_after();
         uint32_t v[COLS];
 #pragma unroll
@@ -506,7 +526,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           m = mn;
           l *= corr;
           if (j > 0) {
-            mbar_wait_bounded(&o_done[s * NB + (g - 1) % NB], ((g - 1) / NB) & 1, dead);
+            wait(&o_done[s * NB + (g - 1) % NB], ((g - 1) / NB) & 1);
             tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < OCOLS; c += 32) {
@@ -542,7 +562,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (vend < kKeys) {
           // the tile's rows of V behind the last key that any stream sees: zeros (both streams write the same zeros)
           const uint32_t kv = kv0 + j;
-          mbar_wait_bounded(&v_full[kv % ST], (kv / ST) & 1, dead);
+          wait(&v_full[kv % ST], (kv / ST) & 1);
           const int r = threadIdx.x & 63;
           if (r >= vend) {
             for (int c = 0; c < CV; ++c)
@@ -571,7 +591,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (p.gate != nullptr && !p.gate_elem && row < rows) inv *= 1.f / (1.f + expf(-__bfloat162float(p.gate[(size_t)(tok + row) * p.ld_gate + head])));
       }
       inv = l > 0.f ? inv / l : 0.f;
-      mbar_wait_bounded(&o_done[s * NB + (g - 1) % NB], ((g - 1) / NB) & 1, dead);
+      wait(&o_done[s * NB + (g - 1) % NB], ((g - 1) / NB) & 1);
       tc_fence_after();
       if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) inv = __int_as_float(0x7fffffff);
       const int col0 = head * DV + (NS == 1 ? half * (DV / 2) : 0);
@@ -620,7 +640,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tc_fence_before();
   }
   __syncthreads();
-  if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) __nanosleep(1000000);   // copies and products in flight end before the CTA's memory goes
+  if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) settle_in_flight();     // before the CTA's memory goes
   if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
@@ -689,6 +709,7 @@ cudaError_t flash_tc_launch(const FlashPrefillArgs& a, cudaStream_t s) {
   FlashTcParams p = {};
   p.block_tables = a.block_tables; p.max_blocks = a.max_blocks; p.cu_seqlens = a.cu_seqlens; p.context_lens = a.context_lens; p.num_seqs = a.num_seqs;
   p.q_heads = a.q_heads; p.kv_heads = a.kv_heads; p.page = a.page; p.box_rows = a.page % kKeys == 0 ? kKeys : a.page; p.lin_stride = -1;
+  p.wait_spins = a.wait_spins;
   p.scale = a.scale; p.softcap = a.softcap; p.out = static_cast<__nv_bfloat16*>(a.out); p.o_ld_t = a.o_ld_t;
   CUtensorMap tq, tk, tv;
   if (!ft_map_q(&tq, a.q, a.dk_, a.q_heads, a.tokens, a.q_ld_h, a.q_ld_t) || !ft_map_2d(&tk, a.kpool, a.dk_, a.pool_rows, a.dk_, p.box_rows) ||

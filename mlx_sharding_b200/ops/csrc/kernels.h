@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "waits.h"
+
 namespace b200 {
 
 // ---- elementwise.cu
@@ -62,6 +64,7 @@ struct FlashPrefillArgs {
   float scale;
   void* out; long long o_ld_t;
   int tokens; float softcap; long long pool_rows;   // (tcgen05 form) query rows, cap on the scores (0: none), pages * kv_heads * page
+  uint32_t wait_spins = kWaitSpins;                 // (tcgen05 form) bound of every wait
 };
 bool flash_prefill_supported(int dk, int dv);
 cudaError_t flash_prefill_launch(const FlashPrefillArgs& a, cudaStream_t s);

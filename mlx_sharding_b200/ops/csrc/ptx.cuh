@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "waits.h"
+
 namespace b200 {
 
 #define B200_DEVICE __device__ __forceinline__
@@ -57,16 +59,24 @@ B200_DEVICE void mbar_wait(uint64_t* bar, uint32_t parity) {
   }
 }
 
-// Bounded wait that marks the CTA dead (a word in shared memory) instead of trapping: every later wait of the CTA then falls through, so the
-// kernel drains, gives its TMEM back and returns with NaN in its results.
-B200_DEVICE void mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
+// Bounded wait that marks the CTA dead (a word in shared memory) instead of trapping.  False: this wait gave up, or another one of the CTA had.
+// The caller then issues and signals nothing more and leaves its loop, so that every role reaches the end of the kernel; there the CTA lets its
+// copies and products in flight land (settle_in_flight), gives its TMEM back and returns.  Its results are void.
+B200_DEVICE bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile uint32_t* dead, uint32_t limit = kWaitSpins) {
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
-    if (++spins > (1u << 20) || *dead != 0u) {
+    if (*dead != 0u) return false;
+    if (++spins > limit) {
       *dead = 1u;
-      return;
+      return false;
     }
   }
+  return true;
+}
+// about a millisecond: a copy or product takes microseconds
+B200_DEVICE void settle_in_flight() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < (1 << 21)) __nanosleep(1000);
 }
 
 // ---------------------------------------------------------------------------------------------- TMA
@@ -220,6 +230,13 @@ B200_DEVICE uint32_t ld_acquire_gpu(const uint32_t* p) {
 }
 B200_DEVICE void named_bar_sync(uint32_t id, uint32_t nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// the same, and whether the predicate holds for every thread of the barrier
+B200_DEVICE bool named_bar_and(uint32_t id, uint32_t nthreads, bool pred) {
+  uint32_t all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbarrier.cta.red.and.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"(id), "r"(nthreads), "r"(pred ? 1u : 0u) : "memory");
+  return all != 0u;
 }
 
 // Programmatic dependent launch (see launch.h): wait for the predecessor grid's memory, then let the successor's
