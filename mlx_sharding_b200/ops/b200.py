@@ -52,6 +52,12 @@ def C():
     return load_extension()
 
 
+def check_waits():
+    """Raises if a wait inside one of this process's kernels has given up since the last look (a load from host memory, no synchronisation: it covers
+    what has completed)."""
+    C().check_waits()
+
+
 def is_available() -> bool:
     return os.path.exists(_SO) and torch.cuda.is_available()
 

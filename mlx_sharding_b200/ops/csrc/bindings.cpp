@@ -46,6 +46,30 @@ void check_rows(const Tensor& t, const char* name) {
   TORCH_CHECK(t.dim() == 2 && t.stride(1) == 1, name, " must be 2-D with a contiguous last dim");
 }
 
+// ---- waits inside kernels ---------------------------------------------------------------------------------------
+// A kernel whose wait gives up writes its code into this word (mapped host memory, so that looking costs the host a load and no synchronisation).
+// The host looks before it launches such a kernel again and where it reads results: the error comes with a later call, as CUDA's own do.
+volatile uint32_t* wait_word() {
+  static uint32_t* word = [] {
+    uint32_t* p = nullptr;
+    CUDA_OK(cudaHostAlloc(reinterpret_cast<void**>(&p), 64, cudaHostAllocMapped | cudaHostAllocPortable));
+    *p = 0;
+    return p;
+  }();
+  return word;
+}
+void check_waits() {
+  const uint32_t code = *wait_word();
+  if (code == 0) return;
+  *wait_word() = 0;
+  TORCH_CHECK(false, "a wait inside a ", code == b200::kWaitPromptAttention ? "prompt attention" : "many-row GEMM",
+              " kernel gave up: what has been computed since the last check is void");
+}
+b200::WaitBound wait_bound(int64_t spins = b200::kWaitSpins) {
+  check_waits();
+  return {(uint32_t)spins, const_cast<uint32_t*>(wait_word())};
+}
+
 // ---- persistent scratch -----------------------------------------------------------------------------------------
 struct Scratch {
   std::vector<Tensor> keep;  // every buffer ever handed out stays alive (graph safety)
@@ -107,7 +131,7 @@ int auto_splits(int rows, int n, int k, bool grouped) {
 // ---- GEMM -------------------------------------------------------------------------------------------------------
 Tensor linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& w2, const c10::optional<Tensor>& residual,
               const c10::optional<Tensor>& bias, int64_t act, double softcap, bool out_fp32, const c10::optional<Tensor>& out_,
-              int64_t splits, int64_t signal_flag_ptr, int64_t signal_value, double act_limit) {
+              int64_t splits, int64_t signal_flag_ptr, int64_t signal_value, double act_limit, int64_t wait_spins) {
   check_bf16(x, "x"); check_bf16(w, "w"); check_rows(x, "x"); check_rows(w, "w");
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t T = x.size(0), K = x.size(1), N = w.size(0);
@@ -116,6 +140,7 @@ Tensor linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& w2,
   TORCH_CHECK(out.dim() == 2 && out.stride(1) == 1 && out.size(0) >= T && out.size(1) == N, "bad out tensor");
   if (T == 0) return out;
   b200::GemmArgs a;
+  a.wait = wait_bound(wait_spins);
   a.x = x.data_ptr(); a.x_rows = T; a.ld_x = x.stride(0);
   a.w = w.data_ptr(); a.ld_w = w.stride(0);
   if (w2.has_value()) { check_bf16(*w2, "w2"); TORCH_CHECK(w2->sizes() == w.sizes() && w2->stride(0) == w.stride(0)); a.w2 = w2->data_ptr(); }
@@ -163,6 +188,7 @@ Tensor grouped_linear(const Tensor& x, const Tensor& w, const c10::optional<Tens
   Tensor out = torch::empty({ep_ret ? 0 : R, N}, x.options().dtype(out_fp32 ? torch::kFloat32 : torch::kBFloat16));
   if (R == 0) return out;
   b200::GemmArgs a;
+  a.wait = wait_bound();
   a.x = x.data_ptr(); a.x_rows = R; a.ld_x = x.stride(0);
   a.w = w.data_ptr(); a.ld_w = K;
   if (w2.has_value()) { check_bf16(*w2, "w2"); TORCH_CHECK(w2->is_contiguous() && w2->sizes() == w.sizes()); a.w2 = w2->data_ptr(); }
@@ -491,7 +517,7 @@ Tensor flash_prefill(const Tensor& q, const Tensor& kpool, const Tensor& vpool, 
   a.block_tables = block_tables.data_ptr<int>(); a.max_blocks = (int)block_tables.size(1);
   a.cu_seqlens = cu_seqlens.data_ptr<int>(); a.context_lens = context_lens.data_ptr<int>();
   a.num_seqs = (int)context_lens.numel(); a.max_tiles = (int)((num_tokens + 63) / 64 + a.num_seqs);
-  a.scale = (float)scale; a.out = out.data_ptr(); a.wait_spins = (uint32_t)wait_spins;
+  a.scale = (float)scale; a.out = out.data_ptr(); a.wait = wait_bound(wait_spins);
   const bool mma_sync = softcap == 0.0 && b200::flash_prefill_supported(a.dk_, a.dv_);
   if (b200::flash_tc_supported(a) && !(mma_sync && flash_short(max_ctx, num_tokens, a.num_seqs, a.q_heads))) {
     LAUNCH_OK(b200::flash_tc_launch(a, cur_stream()));
@@ -548,7 +574,7 @@ Tensor flash_mla(const Tensor& q, const Tensor& kv, const Tensor& pool, const Te
   a.block_tables = block_tables.data_ptr<int>(); a.max_blocks = (int)block_tables.size(1);
   a.cu_seqlens = cu_seqlens.data_ptr<int>(); a.context_lens = context_lens.data_ptr<int>();
   a.num_seqs = (int)context_lens.numel(); a.tokens = (int)q.size(0); a.heads = (int)q.size(1); a.page = (int)pool.size(2);
-  a.lin_stride = lin_stride; a.scale = (float)scale;
+  a.lin_stride = lin_stride; a.scale = (float)scale; a.wait = wait_bound();
   Tensor out = torch::empty({q.size(0), q.size(1) * 128}, q.options());
   a.out = out.data_ptr(); a.o_ld_t = out.stride(0);
   if (a.tokens == 0) return out;
@@ -758,9 +784,10 @@ void copy_signal(const Tensor& src, int64_t dst_ptr, int64_t flag_ptr, int64_t v
                                    reinterpret_cast<unsigned int*>(scratch().get_counters(src.device()).data_ptr<int>()) + 65533,
                                    cur_stream()));
 }
-// allocate the persistent scratch eagerly (must happen before any CUDA-graph capture)
+// allocate the persistent scratch and the word of the waits eagerly (must happen before any CUDA-graph capture)
 void init_scratch(int64_t device, int64_t ws_floats) {
   const c10::cuda::CUDAGuard guard(torch::Device(torch::kCUDA, (int)device));
+  wait_word();
   scratch().get_counters(torch::Device(torch::kCUDA, (int)device));
   scratch().get_ws(ws_floats, torch::Device(torch::kCUDA, (int)device));
 }
@@ -1562,7 +1589,7 @@ Tensor hy_sink_flash(const Tensor& q, const Tensor& kpool, const Tensor& vpool, 
   // few rows over few keys: the mma.sync form (B200, 16 heads, mma.sync / tcgen05: one prompt of 256 tokens 13.8 / 17.5 us, 400 19.6 / 22.0, 600 38.0 / 28.1,
   // three of 200 18.8 / 19.8)
   const bool few = max_ctx > 0 && max_ctx <= 448 && (q.size(0) / 64 + a.B) * a.H <= 3 * sm_count();
-  if (!few && b200::flash_sink_takes(a, pool_rows)) LAUNCH_OK(b200::flash_sink_launch(a, ctx.data_ptr<int>(), pool_rows, (int)q.size(0), cur_stream()));
+  if (!few && b200::flash_sink_takes(a, pool_rows)) LAUNCH_OK(b200::flash_sink_launch(a, ctx.data_ptr<int>(), pool_rows, (int)q.size(0), wait_bound(), cur_stream()));
   else LAUNCH_OK(b200::sink_flash_launch(a, ctx.data_ptr<int>(), (int)((q.size(0) + 63) / 64 + a.B), cur_stream()));
   return out;
 }
@@ -1613,7 +1640,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "mlx_sharding_b200 sm_100a kernels";
   m.def("linear", &linear, py::arg("x"), py::arg("w"), py::arg("w2") = py::none(), py::arg("residual") = py::none(),
         py::arg("bias") = py::none(), py::arg("act") = 0, py::arg("softcap") = 0.0, py::arg("out_fp32") = false,
-        py::arg("out") = py::none(), py::arg("splits") = 0, py::arg("signal_flag_ptr") = 0, py::arg("signal_value") = 0, py::arg("act_limit") = 0.0);
+        py::arg("out") = py::none(), py::arg("splits") = 0, py::arg("signal_flag_ptr") = 0, py::arg("signal_value") = 0, py::arg("act_limit") = 0.0,
+        py::arg("wait_spins") = (int64_t)b200::kWaitSpins);
+  m.def("check_waits", &check_waits);
   m.def("grouped_linear", &grouped_linear, py::arg("x"), py::arg("w"), py::arg("w2") = py::none(), py::arg("expert_offsets"),
         py::arg("max_rows"), py::arg("act") = 0, py::arg("out_fp32") = false, py::arg("row_dst") = py::none(),
         py::arg("signal_peers") = py::none(), py::arg("done_counter") = py::none(), py::arg("expected_rows") = 0,

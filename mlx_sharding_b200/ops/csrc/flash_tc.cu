@@ -64,7 +64,7 @@ struct FlashTcParams {
   const float* sink; const __nv_bfloat16* gate; long long ld_gate;
   int gate_elem, block, window, keep;
   float out_mult;
-  uint32_t wait_spins = kWaitSpins;            // bound of every wait
+  WaitBound wait;
 };
 
 __host__ __device__ constexpr int ft_streams(int dv) { return dv > 128 ? 1 : 2; }
@@ -261,7 +261,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_smem;
   const int total = s_cum[p.num_seqs - 1], items = total * heads;
-  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(bar, parity, dead, p.wait_spins); };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(bar, parity, dead, p.wait.spins); };
   // the i-th item of this CTA, as the producer drew and laid it out; false at the end of the list, or where a wait gave up
   auto item_at = [&](uint32_t i, FlashItem& it) {
     const bool here = wait(&w_full[i % kSlots], (i / kSlots) & 1);
@@ -640,7 +640,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tc_fence_before();
   }
   __syncthreads();
-  if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) settle_in_flight();     // before the CTA's memory goes
+  if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) report_dead(p.wait, kWaitPromptAttention);     // before the CTA's memory goes
   if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
@@ -709,7 +709,7 @@ cudaError_t flash_tc_launch(const FlashPrefillArgs& a, cudaStream_t s) {
   FlashTcParams p = {};
   p.block_tables = a.block_tables; p.max_blocks = a.max_blocks; p.cu_seqlens = a.cu_seqlens; p.context_lens = a.context_lens; p.num_seqs = a.num_seqs;
   p.q_heads = a.q_heads; p.kv_heads = a.kv_heads; p.page = a.page; p.box_rows = a.page % kKeys == 0 ? kKeys : a.page; p.lin_stride = -1;
-  p.wait_spins = a.wait_spins;
+  p.wait = a.wait;
   p.scale = a.scale; p.softcap = a.softcap; p.out = static_cast<__nv_bfloat16*>(a.out); p.o_ld_t = a.o_ld_t;
   CUtensorMap tq, tk, tv;
   if (!ft_map_q(&tq, a.q, a.dk_, a.q_heads, a.tokens, a.q_ld_h, a.q_ld_t) || !ft_map_2d(&tk, a.kpool, a.dk_, a.pool_rows, a.dk_, p.box_rows) ||
@@ -736,7 +736,7 @@ cudaError_t flash_mla_launch(const FlashMlaArgs& a, cudaStream_t s) {
     return cudaErrorInvalidValue;
   FlashTcParams p = {};
   p.block_tables = a.block_tables; p.max_blocks = a.max_blocks; p.cu_seqlens = a.cu_seqlens; p.context_lens = a.context_lens; p.num_seqs = a.num_seqs;
-  p.q_heads = p.kv_heads = a.heads; p.page = a.page; p.box_rows = kKeys; p.lin_stride = a.lin_stride; p.scale = a.scale;
+  p.q_heads = p.kv_heads = a.heads; p.page = a.page; p.box_rows = kKeys; p.lin_stride = a.lin_stride; p.scale = a.scale; p.wait = a.wait;
   p.out = static_cast<__nv_bfloat16*>(a.out); p.o_ld_t = a.o_ld_t;
   CUtensorMap tq, tk, tpe;
   if (!ft_map_q(&tq, a.q, 192, a.heads, a.tokens, a.q_ld_h, a.q_ld_t) || !ft_map_2d(&tk, a.kv, (uint64_t)a.heads * 256, a.kv_rows, a.kv_ld, kKeys) ||
@@ -751,9 +751,10 @@ bool flash_sink_takes(const SinkAttnArgs& a, long long pool_rows) {
          ft_aligned(a.kpool) && ft_aligned(a.vpool) && ft_aligned(a.out) && a.ld_out % 8 == 0 && pool_rows < (1LL << 31) && ft_encode() != nullptr;
 }
 
-cudaError_t flash_sink_launch(const SinkAttnArgs& a, const int* context_lens, long long pool_rows, int tokens, cudaStream_t s) {
+cudaError_t flash_sink_launch(const SinkAttnArgs& a, const int* context_lens, long long pool_rows, int tokens, const WaitBound& wait, cudaStream_t s) {
   if (!flash_sink_takes(a, pool_rows)) return cudaErrorInvalidValue;
   FlashTcParams p = {};
+  p.wait = wait;
   p.block_tables = a.block_tables; p.max_blocks = a.max_blocks; p.cu_seqlens = a.cu; p.context_lens = context_lens; p.num_seqs = a.B;
   p.q_heads = a.H; p.kv_heads = a.G; p.page = a.page; p.box_rows = a.page % kKeys == 0 ? kKeys : a.page; p.lin_stride = -1;
   p.scale = a.scale; p.out = static_cast<__nv_bfloat16*>(a.out); p.o_ld_t = a.ld_out;

@@ -93,7 +93,7 @@ __device__ __forceinline__ int pair_cols(int rows) { return (rows + 31) & ~31; }
 template <bool DUAL, typename OutT>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2, const __grid_constant__ CUtensorMap tmap_x,
-                 const GemmParams p, const int tiles_n, const int tiles_m, const int num_experts) {
+                 const GemmParams p, const int tiles_n, const int tiles_m, const int num_experts, const WaitBound bound) {
   constexpr int ST = pair_stages(DUAL), STAGE = pair_stage_bytes(DUAL), NUM_ACC = DUAL ? 1 : 2;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -147,17 +147,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const uint32_t tmem_base = *tmem_base_smem;
   const int total = num_experts > 0 ? s_cum[num_experts] : tiles_n * tiles_m;
   const int kb_total = (p.k + kBlockK - 1) / kBlockK;
+  // A CTA whose wait gives up signals nothing more; its neighbour's waits then run out by themselves, and both meet at the end.
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(bar, parity, dead, bound.spins); };
+  bool alive = true;
 
   if (warp == 0) {
     // ============================================================== TMA producer: own weight rows, own half of the tokens
     if (elect_one()) {
       uint32_t it = 0;
-      for (int t = cid; t < total; t += ncl) {
+      for (int t = cid; alive && t < total; t += ncl) {
         const PairTile ti = pair_tile(p, s_cum, s_off, num_experts, t, tiles_n, tiles_m);
         const int x_row = ti.row_base + (int)rank * (pair_cols(ti.rows) >> 1), w_row = ti.w_row + (int)rank * kTileM;
         for (int kb = 0; kb < kb_total; ++kb, ++it) {
           const uint32_t s = it % ST, ph = (it / ST) & 1;
-          mbar_wait_bounded(&empty_bar[s], ph ^ 1, dead);
+          alive = wait(&empty_bar[s], ph ^ 1);
+          if (!alive) break;
           if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * STAGE);
           const uint32_t st = smem_u32(smem + s * STAGE), bar = mapa_shared(smem_u32(&full_bar[s]), 0);
           const int kc = kb * kBlockK;
@@ -167,22 +171,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
       }
       // the leader's commits to this CTA's barriers have all arrived before the CTA may go
-      for (int i = 0; i < ST; ++i, ++it) mbar_wait_bounded(&empty_bar[it % ST], ((it / ST) & 1) ^ 1, dead);
+      for (int i = 0; alive && i < ST; ++i, ++it) alive = wait(&empty_bar[it % ST], ((it / ST) & 1) ^ 1);
     }
   } else if (warp == 1) {
     // ============================================================== MMA issuer of the pair
     if (rank == 0 && elect_one()) {
       uint32_t it = 0, tc = 0;
-      for (int t = cid; t < total; t += ncl, ++tc) {
+      for (int t = cid; alive && t < total; t += ncl, ++tc) {
         const PairTile ti = pair_tile(p, s_cum, s_off, num_experts, t, tiles_n, tiles_m);
         const uint32_t idesc = umma_idesc_bf16(2 * kTileM, (uint32_t)pair_cols(ti.rows));
         const uint32_t ab = tc % NUM_ACC, aph = (tc / NUM_ACC) & 1;
-        mbar_wait_bounded(&tempty_bar[ab], aph ^ 1, dead);
+        alive = wait(&tempty_bar[ab], aph ^ 1);
         tc_fence_after();
         const uint32_t acc = tmem_base + ab * kPairTok;
-        for (int kb = 0; kb < kb_total; ++kb, ++it) {
+        for (int kb = 0; alive && kb < kb_total; ++kb, ++it) {
           const uint32_t s = it % ST, ph = (it / ST) & 1;
-          mbar_wait_bounded(&full_bar[s], ph, dead);
+          alive = wait(&full_bar[s], ph);
+          if (!alive) break;
           tc_fence_after();
           const uint32_t a0 = smem_u32(smem + s * STAGE);
           const uint64_t ad = umma_desc_sw128(a0), ad2 = umma_desc_sw128(a0 + kATileBytes), bd = umma_desc_sw128(a0 + kATileBytes * (DUAL ? 2 : 1));
@@ -193,7 +198,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           }
           pair_commit(&empty_bar[s]);
         }
-        pair_commit(&tfull_bar[ab]);
+        if (alive) pair_commit(&tfull_bar[ab]);
       }
     }
   } else if (warp >= 4) {
@@ -207,7 +212,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const int f = ti.n0 + (int)rank * kTileM + q * 32 + lane;
       const bool f_ok = f < p.n;
       const float bias = (p.bias != nullptr && f_ok) ? __bfloat162float(p.bias[f]) : 0.0f;
-      mbar_wait_bounded(&tfull_bar[ab], aph, dead);
+      if (!__all_sync(0xffffffffu, wait(&tfull_bar[ab], aph))) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + lane_addr + ab * kPairTok;
 #pragma unroll 1
@@ -264,16 +269,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) {
-    // a wait ran out: copies and products in flight end first, and the first result of the tile list says so
-    __nanosleep(1000000);
-    if (threadIdx.x == 0 && cid < total) {
-      const PairTile ti = pair_tile(p, s_cum, s_off, num_experts, cid, tiles_n, tiles_m);
-      if (sizeof(OutT) == 2) reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)ti.row_base * p.ld_out + ti.n0] = __float2bfloat16_rn(__int_as_float(0x7fffffff));
-      else reinterpret_cast<float*>(p.out)[(size_t)ti.row_base * p.ld_out + ti.n0] = __int_as_float(0x7fffffff);
-    }
-    __syncthreads();
-  }
+  if (*reinterpret_cast<volatile uint32_t*>(dead) != 0u) report_dead(bound, kWaitPairGemm);
   cluster_sync_all();                                                       // nobody reads or signals this CTA any more
   if (warp == 1) {
     tc_fence_after();
@@ -285,7 +281,7 @@ namespace {
 
 template <bool DUAL, typename OutT>
 cudaError_t pair_launch_one(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx, const GemmParams& p, int tiles_n, int tiles_m, int experts,
-                            long long tiles, cudaStream_t stream) {
+                            long long tiles, const WaitBound& wait, cudaStream_t stream) {
   constexpr int smem = pair_smem(DUAL);
   static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
   auto kern = gemm_pair_kernel<DUAL, OutT>;
@@ -304,7 +300,7 @@ cudaError_t pair_launch_one(const CUtensorMap& tw, const CUtensorMap& tw2, const
     fit = n > 0 ? n : 1;
   }
   const int clusters = static_cast<int>(std::min<long long>(tiles, fit));
-  (void)launch_pdl_cluster(kern, dim3(2 * clusters), dim3(kPairThreads), smem, stream, dim3(2), tw, tw2, tx, p, tiles_n, tiles_m, experts);
+  (void)launch_pdl_cluster(kern, dim3(2 * clusters), dim3(kPairThreads), smem, stream, dim3(2), tw, tw2, tx, p, tiles_n, tiles_m, experts, wait);
   return cudaGetLastError();
 }
 
@@ -335,9 +331,9 @@ cudaError_t gemm_pair_launch(const GemmArgs& a, cudaStream_t stream) {
   const int tiles_n = (a.n + kPairFeat - 1) / kPairFeat, tiles_m = (a.max_rows + kPairTok - 1) / kPairTok;
   const long long most = static_cast<long long>(tiles_n) * tiles_m * (grouped ? a.num_experts : 1);
   const int experts = grouped ? a.num_experts : 0;
-  if (a.out_fp32) return pair_launch_one<false, float>(tw, tw2, tx, p, tiles_n, tiles_m, experts, most, stream);
-  if (dual) return pair_launch_one<true, __nv_bfloat16>(tw, tw2, tx, p, tiles_n, tiles_m, experts, most, stream);
-  return pair_launch_one<false, __nv_bfloat16>(tw, tw2, tx, p, tiles_n, tiles_m, experts, most, stream);
+  if (a.out_fp32) return pair_launch_one<false, float>(tw, tw2, tx, p, tiles_n, tiles_m, experts, most, a.wait, stream);
+  if (dual) return pair_launch_one<true, __nv_bfloat16>(tw, tw2, tx, p, tiles_n, tiles_m, experts, most, a.wait, stream);
+  return pair_launch_one<false, __nv_bfloat16>(tw, tw2, tx, p, tiles_n, tiles_m, experts, most, a.wait, stream);
 }
 
 }  // namespace b200

@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "waits.h"
+
 namespace b200 {
 
 // kActClampedGlu (two-weight form only): g' = min(g, act_limit), u' = clamp(u, +-act_limit), y = g' sigmoid(1.702 g') (u' + 1)
@@ -84,6 +86,7 @@ struct GemmArgs {
   const void* w_sf = nullptr; const void* w2_sf = nullptr; const void* x_sf = nullptr;
   bool persistent = true;                 // splits == 1: persistent kernel (gemm_persistent.cu)
   bool cluster_splitk = true;             // prefer the DSMEM reduction when it applies (decode shapes)
+  WaitBound wait;                         // of the waits of gemm_pair.cu
   int q_bits = 0, q_group = 64;
   const void* q_scales_t = nullptr; const void* q_biases_t = nullptr;
   const void* q_scales2_t = nullptr; const void* q_biases2_t = nullptr;

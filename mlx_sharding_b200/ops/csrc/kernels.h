@@ -64,7 +64,7 @@ struct FlashPrefillArgs {
   float scale;
   void* out; long long o_ld_t;
   int tokens; float softcap; long long pool_rows;   // (tcgen05 form) query rows, cap on the scores (0: none), pages * kv_heads * page
-  uint32_t wait_spins = kWaitSpins;                 // (tcgen05 form) bound of every wait
+  WaitBound wait;                                   // (tcgen05 form) of every wait
 };
 bool flash_prefill_supported(int dk, int dv);
 cudaError_t flash_prefill_launch(const FlashPrefillArgs& a, cudaStream_t s);
@@ -83,6 +83,7 @@ struct FlashMlaArgs {
   long long lin_stride;                          // row of a sequence's position 0 in `kv`: seq * lin_stride, or (< 0) its first token's row
   float scale;
   void* out; long long o_ld_t;                   // bf16 [T, heads * 128]
+  WaitBound wait;
 };
 bool flash_mla_supported(int num_seqs);
 cudaError_t flash_mla_launch(const FlashMlaArgs& a, cudaStream_t s);

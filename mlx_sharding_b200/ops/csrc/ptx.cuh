@@ -61,8 +61,8 @@ B200_DEVICE void mbar_wait(uint64_t* bar, uint32_t parity) {
 
 // Bounded wait that marks the CTA dead (a word in shared memory) instead of trapping.  False: this wait gave up, or another one of the CTA had.
 // The caller then issues and signals nothing more and leaves its loop, so that every role reaches the end of the kernel; there the CTA lets its
-// copies and products in flight land (settle_in_flight), gives its TMEM back and returns.  Its results are void.
-B200_DEVICE bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile uint32_t* dead, uint32_t limit = kWaitSpins) {
+// copies and products in flight land and tells the host (report_dead), gives its TMEM back and returns.  What the launch has written is void.
+B200_DEVICE bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile uint32_t* dead, uint32_t limit) {
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
     if (*dead != 0u) return false;
@@ -73,10 +73,14 @@ B200_DEVICE bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile uint
   }
   return true;
 }
-// about a millisecond: a copy or product takes microseconds
-B200_DEVICE void settle_in_flight() {
+// after the CTA's last barrier: about a millisecond (a copy or product takes microseconds), and the word that the host reads
+B200_DEVICE void report_dead(const WaitBound& w, uint32_t code) {
   const long long t0 = clock64();
   while (clock64() - t0 < (1 << 21)) __nanosleep(1000);
+  if (threadIdx.x == 0 && w.error != nullptr) {
+    *reinterpret_cast<volatile uint32_t*>(w.error) = code;
+    __threadfence_system();
+  }
 }
 
 // ---------------------------------------------------------------------------------------------- TMA

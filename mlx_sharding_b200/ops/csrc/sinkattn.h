@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "waits.h"
+
 namespace b200 {
 struct SinkAttnArgs {
   const float* q;                           // fp32 [T, H, D] (normed, rotated)
@@ -36,6 +38,6 @@ bool sink_flash_supported(int D, int V);
 int sink_flash_bias_max();                  // longest distance table (slopes and a table together: the vector form alone)
 // ... and on tcgen05 (flash_tc.cu): heads of 64 / 128, no terms by distance, pages that TMA boxes fit; pool_rows = pages * G * page
 bool flash_sink_takes(const SinkAttnArgs& a, long long pool_rows);
-cudaError_t flash_sink_launch(const SinkAttnArgs& a, const int* context_lens, long long pool_rows, int tokens, cudaStream_t s);
+cudaError_t flash_sink_launch(const SinkAttnArgs& a, const int* context_lens, long long pool_rows, int tokens, const WaitBound& wait, cudaStream_t s);
 cudaError_t sink_flash_launch(const SinkAttnArgs& a, const int* context_lens, int max_tiles, cudaStream_t s);
 }  // namespace b200

@@ -198,6 +198,10 @@ def moe_route(x: torch.Tensor, gate_w: torch.Tensor, top_k: int, method: str = "
     return order.to(torch.int32), w
 
 
+def check_waits():
+    """Backend hook: the CUDA backend raises here when a wait inside a kernel has given up."""
+
+
 # ------------------------------------------------------------------------------------------ K11
 def run_aside(fn, lane: int = 0):
     """Backend hook: independent work that the CUDA backend forks onto a side stream (``lane``: which of them) runs inline here."""

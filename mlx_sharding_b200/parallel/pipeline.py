@@ -70,7 +70,9 @@ class StageExecutor:
     @torch.inference_mode()
     def sample(self, logits: torch.Tensor, inp_params, contexts) -> StepOutput:
         so = self.sampler(logits, inp_params, contexts)
-        return StepOutput(so.tokens.tolist(), so.logprobs.tolist(),
+        toks = so.tokens.tolist()
+        self.model.ops.check_waits()
+        return StepOutput(toks, so.logprobs.tolist(),
                           None if so.top_ids is None else so.top_ids.tolist(),
                           None if so.top_logprobs is None else so.top_logprobs.tolist())
 
@@ -136,10 +138,11 @@ class StepRunner:
     def run(self, wire: np.ndarray, group: int, x_local: Optional[torch.Tensor] = None):
         """``wire`` = ``[header | step block]`` (int32).  Returns the stage output: hidden ``[T, H]`` or, on the last stage, the
         result message (device uint8 tensor)."""
+        self._phase, self._x_local = 0, x_local
+        self.model.ops.check_waits()     # of an earlier step of this stage (a stage that is not the last never waits for its own)
         lay, _ = unpack_header(wire)
         blk = wire[HEADER_WORDS:HEADER_WORDS + lay.size]
         mq, mctx = int(blk[lay.meta + 2]), int(blk[lay.meta + 3])
-        self._phase, self._x_local = 0, x_local
         with self.stage.timer.measure():
             if self.gcache.enabled and mq == 1 and lay.T == lay.B and x_local is None:
                 e = self.gcache.entry(lay, mctx, group)
@@ -232,6 +235,7 @@ class LocalPipeline:
             x = r.run(wire, inp.group, x_local=None if x is None else x.to(r.dev))
         rl = ResultLayout(lay.B, lay.k)
         host = _fetch(x)
+        self.stages[0].model.ops.check_waits()
         self.d2h_bytes += rl.nbytes
         return _step_output(parse_result(host, rl, self._seq), inp.meta.num_seqs)
 
@@ -530,6 +534,7 @@ class ChainPipeline:
             self._outstanding.remove(handle)
         except ValueError:
             pass
+        self.stage.model.ops.check_waits()
         self._raise_if_failed()
         if self.plane.failed():
             self._dead = "P2P flag wait timed out: a pipeline stage is not responding"

@@ -65,3 +65,27 @@ def test_cancel_releases_pages_and_rejects_bad_requests():
     eng.drain()
     assert r.finished and r.finish_reason == "cancelled" and len(r.output) < 40
     assert eng.table.alloc.num_free == 31
+
+
+def test_wait_that_gave_up_fails_the_requests_and_the_engine_goes_on(monkeypatch):
+    """A backend that reports a wait given up inside a kernel (the CUDA backend's ``check_waits``): the step's requests get the error, the next ones run."""
+    (m,) = _stages([(0, 4)])
+    eng = LLMEngine(LocalPipeline.from_models([m], 32, 16), 32, 16)
+    want = eng.generate([1, 2, 3], SamplingParams(temperature=0.0), max_tokens=3)
+    looks = []
+
+    def gave_up():
+        looks.append(1)
+        if len(looks) == 4:                    # (a look before each step and one where its result is read)
+            raise RuntimeError("a wait inside a kernel gave up")
+
+    monkeypatch.setattr(m.ops, "check_waits", gave_up)
+    eng.start()
+    try:
+        r = eng.submit([1, 2, 3], SamplingParams(temperature=0.0), max_tokens=8)
+        with pytest.raises(RuntimeError, match="gave up"):
+            list(r)
+        assert len(looks) == 4 and r.finished and len(r.output) == 1 and eng.table.alloc.num_free == 31
+        assert eng.generate([1, 2, 3], SamplingParams(temperature=0.0), max_tokens=3) == want
+    finally:
+        eng.shutdown()

@@ -1,4 +1,4 @@
-"""Bounded waits inside kernels: a kernel whose waits run out gives its memory back and returns, and the next launch is right."""
+"""Bounded waits inside kernels: a kernel whose waits run out gives its memory back and returns, the host gets an error, and the next launch is right."""
 import pytest
 import torch
 
@@ -34,4 +34,39 @@ def test_prompt_attention_returns(C, H, Hk, dk, dv):
     for spins in (0, 3, 20):                                     # a wait gives up at its first failed looks: in every phase of the kernel
         call(wait_spins=spins)
         torch.cuda.synchronize()
+        if spins == 0:                                           # (a few looks may be enough)
+            with pytest.raises(RuntimeError, match="prompt attention"):
+                C.check_waits()
+        else:
+            try:
+                C.check_waits()
+            except RuntimeError:
+                pass
     assert torch.equal(call(), want)
+    torch.cuda.synchronize()
+    C.check_waits()
+
+
+# one accumulator set and two, fp32 results; several tiles per pair
+@pytest.mark.parametrize("dual,fp32", [(False, False), (True, False), (False, True)])
+def test_many_row_gemm_returns(C, dual, fp32):
+    g = torch.Generator(device="cuda").manual_seed(0)
+    rnd = lambda *s: (torch.randn(*s, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    x, w, w2 = rnd(5000, 1024), rnd(4096, 1024), rnd(4096, 1024) if dual else None
+    call = lambda **kw: C.linear(x, w, w2, act=1 if dual else 0, out_fp32=fp32, **kw)
+    want = call()
+    torch.cuda.synchronize()
+    for spins in (0, 3, 20):
+        call(wait_spins=spins)
+        torch.cuda.synchronize()
+        if spins == 0:
+            with pytest.raises(RuntimeError, match="GEMM"):
+                call()                                           # a later launch says so, and is not made
+        else:
+            try:
+                C.check_waits()
+            except RuntimeError:
+                pass
+    assert torch.equal(call(), want)
+    torch.cuda.synchronize()
+    C.check_waits()
