@@ -42,7 +42,7 @@ def load_extension(build_if_missing: bool = False):
     spec.loader.exec_module(mod)
     _C = mod
     if torch.cuda.is_available():
-        # persistent scratch (split-K / attention-split workspace, tile tickets) must exist before any
+        # the scratch of captured launches (split-K / attention-split workspace, tickets) must exist before any
         # CUDA-graph capture
         mod.init_scratch(torch.cuda.current_device(), 32 << 20)
     return _C
@@ -196,6 +196,8 @@ def _token_seq(meta: BatchMeta) -> torch.Tensor:
 
 
 def paged_attention(q, kpool, vpool, meta: BatchMeta, scale: float, softcap: float = 0.0):
+    """Causal attention over the paged cache.  Long contexts are split over CTAs that meet through tickets and partial sums: eager calls may run on
+    several streams at once; captured calls share one set of them, so graphs that hold some are replayed one at a time."""
     c = C()
     softcap = float(softcap or 0.0)
     if meta.max_q_len > 1 and c.flash_prefill_takes(q, kpool, vpool, softcap, int(meta.num_seqs), int(meta.max_ctx_len)):
@@ -233,8 +235,8 @@ def run_aside(fn, lane: int = 0) -> _Join:
     """Run ``fn()`` on this device's side stream (``lane``: which of them), forked from the current stream (event record / wait, so it is also legal
     inside CUDA-graph capture and becomes a parallel branch of the graph).  Used to run the shared-expert GEMMs of a
     DeepSeek MoE block concurrently with the router / permutation / expert all-to-all, which do not depend on them.
-    ``fn`` must write its result into a tensor allocated *before* the fork.  Split-K products share one workspace: keep them on one
-    stream."""
+    ``fn`` must write its result into a tensor allocated *before* the fork.  Inside a capture, split-K products and decode attention share
+    one workspace (eager ones have one per stream): keep them on one branch of the graph."""
     cur = torch.cuda.current_stream()
     key = (cur.device.index, lane) if lane else cur.device.index
     side = _side_streams.get(key)

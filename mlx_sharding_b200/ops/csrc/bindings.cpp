@@ -1,11 +1,15 @@
 // PyTorch bindings for the sm_100a kernels.  Everything launches on the current torch CUDA stream so
-// the ops compose with torch.cuda.CUDAGraph capture; scratch buffers are process-lifetime (never freed,
-// never moved once handed to a kernel) so captured graphs stay valid.
+// the ops compose with torch.cuda.CUDAGraph capture; scratch buffers handed to captured launches are never
+// freed or moved, so graphs stay valid.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <map>
+#include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "gemm_tcgen05.h"
@@ -71,29 +75,39 @@ b200::WaitBound wait_bound(int64_t spins = b200::kWaitSpins) {
 }
 
 // ---- persistent scratch -----------------------------------------------------------------------------------------
+// The CTAs of a launch hand each other partial sums and tickets through these buffers, so launches that may run at the same time do not share
+// them: a set per stream for eager launches, and one set per device for captured ones, whose graphs hold its addresses (so captured steps of a
+// device are replayed one at a time, and branches of one graph that need it stay on one stream: ops/b200.py::run_aside).
 struct Scratch {
-  std::vector<Tensor> keep;  // every buffer ever handed out stays alive (graph safety)
+  bool captured = false;
+  std::vector<Tensor> keep;  // captured: every buffer ever handed out stays alive
   Tensor ws;                 // fp32 split-K / attention-split workspace
   Tensor counters;           // uint32 tile tickets (self-resetting) + done counters
   Tensor get_ws(int64_t floats, const torch::Device& dev) {
     if (!ws.defined() || ws.numel() < floats) {
-      int64_t n = std::max<int64_t>(floats, 16 << 20);
-      ws = torch::empty({n}, torch::dtype(torch::kFloat32).device(dev));
-      keep.push_back(ws);
+      int64_t n = std::max<int64_t>(floats, 4 << 20);
+      ws = torch::empty({n}, torch::dtype(torch::kFloat32).device(dev));   // (eager: the smaller one goes back to the allocator in the order of its stream)
+      if (captured) keep.push_back(ws);
     }
     return ws;
   }
   Tensor get_counters(const torch::Device& dev) {
-    if (!counters.defined()) {
-      counters = torch::zeros({1 << 16}, torch::dtype(torch::kInt32).device(dev));
-      keep.push_back(counters);
-    }
+    if (!counters.defined()) counters = torch::zeros({1 << 16}, torch::dtype(torch::kInt32).device(dev));
     return counters;
   }
 };
-Scratch& scratch() {
-  static Scratch s;
+Scratch& scratch_of(int device, cudaStream_t stream, bool captured) {
+  static std::mutex mutex;
+  static std::map<std::tuple<int, cudaStream_t, bool>, Scratch> sets;      // (references stay valid)
+  std::lock_guard<std::mutex> lock(mutex);
+  Scratch& s = sets[{device, captured ? nullptr : stream, captured}];
+  s.captured = captured;
   return s;
+}
+// of the current device and stream
+Scratch& scratch() {
+  const auto s = at::cuda::getCurrentCUDAStream();
+  return scratch_of((int)s.device_index(), s.stream(), c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None);
 }
 
 int sm_count() {
@@ -784,12 +798,14 @@ void copy_signal(const Tensor& src, int64_t dst_ptr, int64_t flag_ptr, int64_t v
                                    reinterpret_cast<unsigned int*>(scratch().get_counters(src.device()).data_ptr<int>()) + 65533,
                                    cur_stream()));
 }
-// allocate the persistent scratch and the word of the waits eagerly (must happen before any CUDA-graph capture)
+// allocate the scratch of captured launches and the word of the waits (must happen before any CUDA-graph capture)
 void init_scratch(int64_t device, int64_t ws_floats) {
   const c10::cuda::CUDAGuard guard(torch::Device(torch::kCUDA, (int)device));
   wait_word();
-  scratch().get_counters(torch::Device(torch::kCUDA, (int)device));
-  scratch().get_ws(ws_floats, torch::Device(torch::kCUDA, (int)device));
+  Scratch& s = scratch_of((int)device, nullptr, true);
+  s.get_counters(torch::Device(torch::kCUDA, (int)device));
+  s.get_ws(ws_floats, torch::Device(torch::kCUDA, (int)device));
+  CUDA_OK(cudaStreamSynchronize(cur_stream()));                            // the tickets are zero for graphs on any stream
 }
 void advance_meta(Tensor positions, Tensor context_lens, Tensor slots, const Tensor& block_tables, int64_t page) {
   TORCH_CHECK(positions.scalar_type() == torch::kInt32 && block_tables.scalar_type() == torch::kInt32 && block_tables.is_contiguous());
