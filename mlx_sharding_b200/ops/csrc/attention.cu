@@ -306,6 +306,8 @@ int paged_attention_splits(int T, int kv_heads, int dk, int dv, int max_ctx, int
 
 cudaError_t paged_attention_launch(const PagedAttnArgs& a, cudaStream_t s) {
   if (a.T == 0) return cudaSuccess;
+  const uintptr_t kv = reinterpret_cast<uintptr_t>(a.kpool) | reinterpret_cast<uintptr_t>(a.vpool);
+  if ((kv & 15) || (reinterpret_cast<uintptr_t>(a.q) & 3)) return cudaErrorInvalidValue;      // cp.async of 16 bytes; queries in pairs
   if ((a.q_ld_t % 2) || (a.q_ld_h % 2) || a.nsplit < 1 || a.nsplit > 64) return cudaErrorInvalidValue;
   if (a.nsplit > 1 && (a.part_acc == nullptr || a.part_ml == nullptr || a.tickets == nullptr)) return cudaErrorInvalidValue;
   const int G = a.q_heads / a.kv_heads;

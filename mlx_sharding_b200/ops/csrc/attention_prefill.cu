@@ -9,8 +9,8 @@
 // double buffered with cp.async straight from the page pool into padded (bank-conflict-free) shared memory.
 // S = QK^T and O += PV run on the tensor cores through warp-level mma.m16n8k16 (bf16 in, fp32 accumulate) with
 // the FA-2 register pipeline (S accumulators are re-used as the A operand of PV); softmax is online in
-// registers with exp2.  The plain form takes what flash_tc.cu (tcgen05, TMA) does not: pages that no TMA box fits (8, 24, 48, ...) and
-// rows that are not 16-byte aligned.
+// registers with exp2.  The plain form takes what flash_tc.cu (tcgen05, TMA) does not: pages that no TMA box fits (8, 24, 48, ...), query
+// rows that are not 16-byte aligned (pools always are), more than 512 sequences; and a few short prompts, where it starts sooner.
 //
 // SINK form (attention of sinkattn.cu for long portions that flash_tc.cu does not take: terms by distance, head sizes other than 64 / 128): keys visible inside blocks of positions or a sliding window beside kept first
 // tokens (only tiles with visible keys are walked), a bias by distance on the scores (DIST 1: slope per head, 2: table per head, in shared
@@ -331,6 +331,8 @@ cudaError_t launch_prefill(const FlashPrefillArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+bool pools_aligned(const void* k, const void* v) { return ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) == 0; }   // cp.async of 16 bytes
+
 constexpr int kBiasMax = 8192;               // entries of a distance table that shared memory takes
 
 template <int DK, int DV, int DIST>
@@ -370,6 +372,7 @@ bool flash_prefill_supported(int dk, int dv) {
 
 cudaError_t flash_prefill_launch(const FlashPrefillArgs& a, cudaStream_t s) {
   if (a.num_seqs == 0 || a.max_tiles == 0) return cudaSuccess;
+  if (!pools_aligned(a.kpool, a.vpool) || (reinterpret_cast<uintptr_t>(a.q) & 3)) return cudaErrorInvalidValue;
   if ((a.q_ld_t % 2) || (a.q_ld_h % 2)) return cudaErrorInvalidValue;
   if (a.dk_ == 192 && a.dv_ == 128) return launch_prefill<192, 128>(a, s);
   if (a.dk_ == 128 && a.dv_ == 128) return launch_prefill<128, 128>(a, s);
@@ -381,6 +384,7 @@ bool sink_flash_supported(int D, int V) { return D % 8 == 0 && V % 8 == 0 && D >
 int sink_flash_bias_max() { return kBiasMax; }
 
 cudaError_t sink_flash_launch(const SinkAttnArgs& a, const int* context_lens, int max_tiles, cudaStream_t s) {
+  if (!pools_aligned(a.kpool, a.vpool)) return cudaErrorInvalidValue;
   if (!sink_flash_supported(a.D, a.V) || a.ld_out % 2 != 0 || a.keep < 0) return cudaErrorInvalidValue;
   if (a.B == 0 || max_tiles == 0) return cudaSuccess;
   if (a.slopes != nullptr && a.bias != nullptr) return cudaErrorInvalidValue;

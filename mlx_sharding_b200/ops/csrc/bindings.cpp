@@ -50,6 +50,8 @@ void check_rows(const Tensor& t, const char* name) {
   TORCH_CHECK(t.dim() == 2 && t.stride(1) == 1, name, " must be 2-D with a contiguous last dim");
 }
 
+bool on16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+
 // ---- waits inside kernels ---------------------------------------------------------------------------------------
 // A kernel whose wait gives up writes its code into this word (mapped host memory, so that looking costs the host a load and no synchronisation).
 // The host looks before it launches such a kernel again and where it reads results: the error comes with a later call, as CUDA's own do.
@@ -387,6 +389,7 @@ void kv_write(const Tensor& k, const Tensor& v, Tensor kpool, Tensor vpool, cons
   check_bf16(k, "k"); check_bf16(v, "v"); check_bf16(kpool, "kpool"); check_bf16(vpool, "vpool");
   TORCH_CHECK(k.dim() == 3 && v.dim() == 3 && k.stride(2) == 1 && v.stride(2) == 1 && kpool.is_contiguous() && vpool.is_contiguous());
   TORCH_CHECK(slots.scalar_type() == torch::kInt32);
+  TORCH_CHECK(on16(k) && on16(v) && on16(kpool) && on16(vpool), "kv_write: keys, values and pools must start on 16 bytes");
   const c10::cuda::CUDAGuard guard(k.device());
   LAUNCH_OK(b200::kv_write_launch(k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0), v.stride(1), kpool.data_ptr(),
                                 vpool.data_ptr(), slots.data_ptr<int>(), (int)k.size(1), (int)k.size(2), (int)v.size(2),
@@ -460,16 +463,20 @@ Tensor linear_fp8(const Tensor& xq, const Tensor& xsf, const Tensor& wq, const T
 }
 
 // ---- attention --------------------------------------------------------------------------------------------------
-Tensor paged_attention(const Tensor& q, const Tensor& kpool, const Tensor& vpool, const Tensor& block_tables, const Tensor& positions,
+// The attention kernels copy keys and values 16 bytes at a time: a pool itself, or a copy where it is a view at an odd offset.
+Tensor pool16(const Tensor& pool) { return on16(pool) ? pool : pool.clone(); }
+
+Tensor paged_attention(const Tensor& q, const Tensor& kpool_, const Tensor& vpool_, const Tensor& block_tables, const Tensor& positions,
                        const Tensor& token_seq, double scale, double softcap, int64_t max_ctx) {
-  check_bf16(q, "q"); check_bf16(kpool, "kpool"); check_bf16(vpool, "vpool");
-  TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && kpool.is_contiguous() && vpool.is_contiguous());
+  check_bf16(q, "q"); check_bf16(kpool_, "kpool"); check_bf16(vpool_, "vpool");
+  TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && kpool_.is_contiguous() && vpool_.is_contiguous());
   TORCH_CHECK(block_tables.scalar_type() == torch::kInt32 && block_tables.is_contiguous() && positions.scalar_type() == torch::kInt32 &&
               token_seq.scalar_type() == torch::kInt32);
   const c10::cuda::CUDAGuard guard(q.device());
-  const int T = (int)q.size(0), Hq = (int)q.size(1), Hk = (int)kpool.size(1), dv = (int)vpool.size(3);
+  const int T = (int)q.size(0), Hq = (int)q.size(1), Hk = (int)kpool_.size(1), dv = (int)vpool_.size(3);
   Tensor out = torch::empty({T, Hq, dv}, q.options());
   if (T == 0) return out;
+  const Tensor kpool = pool16(kpool_), vpool = pool16(vpool_);
   b200::PagedAttnArgs a;
   a.q = q.data_ptr(); a.q_ld_t = q.stride(0); a.q_ld_h = q.stride(1);
   a.kpool = kpool.data_ptr(); a.vpool = vpool.data_ptr();
@@ -518,13 +525,14 @@ bool flash_prefill_takes(const Tensor& q, const Tensor& kpool, const Tensor& vpo
   return (b200::flash_tc_supported(a) && (mma_sync || max_ctx > 32 || (max_ctx > 16 && a.tokens > 128))) || (softcap == 0.0 && b200::flash_prefill_supported(a.dk_, a.dv_));
 }
 
-Tensor flash_prefill(const Tensor& q, const Tensor& kpool, const Tensor& vpool, const Tensor& block_tables, const Tensor& cu_seqlens,
+Tensor flash_prefill(const Tensor& q, const Tensor& kpool_, const Tensor& vpool_, const Tensor& block_tables, const Tensor& cu_seqlens,
                      const Tensor& context_lens, double scale, int64_t num_tokens, double softcap, int64_t max_ctx, int64_t wait_spins) {
-  check_bf16(q, "q"); check_bf16(kpool, "kpool"); check_bf16(vpool, "vpool");
-  TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && kpool.is_contiguous() && vpool.is_contiguous());
+  check_bf16(q, "q"); check_bf16(kpool_, "kpool"); check_bf16(vpool_, "vpool");
+  TORCH_CHECK(q.dim() == 3 && q.stride(2) == 1 && kpool_.is_contiguous() && vpool_.is_contiguous());
   TORCH_CHECK(block_tables.scalar_type() == torch::kInt32 && block_tables.is_contiguous() && cu_seqlens.scalar_type() == torch::kInt32 &&
               context_lens.scalar_type() == torch::kInt32);
   const c10::cuda::CUDAGuard guard(q.device());
+  const Tensor kpool = pool16(kpool_), vpool = pool16(vpool_);
   b200::FlashPrefillArgs a = flash_args(q, kpool, vpool, softcap);
   Tensor out = torch::empty({a.tokens, a.q_heads, a.dv_}, q.options());
   if (a.tokens == 0) return out;

@@ -227,3 +227,18 @@ def test_sink_flash(B, H, Hk, d, page, block, window, keep, gate, sink):
         assert ((got - ref).abs() <= ref.abs() * 1.01 * 2 ** -8 + mag * 2 ** -8 + 2e-4).all(), float((got - ref).abs().max())
         at += n
     assert (out[:, :8] == 0).all() and (out[:, 8 + H * d:] == 0).all()
+
+
+@pytest.mark.parametrize("q_lens,ctx0", [([1, 1, 1], [3, 900, 64]), ([40, 129], [0, 70])])
+@pytest.mark.parametrize("H,Hk,dk,dv,cap", [(8, 2, 128, 128, 0.0), (4, 2, 256, 256, 50.0), (2, 2, 192, 128, 0.0)])
+def test_pools_at_odd_offsets(B, H, Hk, dk, dv, cap, q_lens, ctx0):
+    """Pools that are views four bytes into a buffer: the kernels copy 16 bytes at a time."""
+    meta, tables, kpool, vpool, rnd = paged(q_lens, ctx0, Hk, dk, dv, 64)
+    at_odd = lambda p: torch.empty(p.numel() + 2, dtype=p.dtype, device="cuda")[2:].view(p.shape).copy_(p)
+    q = rnd(meta.num_tokens, H, dk)
+    got = B.paged_attention(q, at_odd(kpool), at_odd(vpool), meta, dk ** -0.5, cap).double()
+    ref, mag = exact(q, kpool, vpool, tables, q_lens, ctx0, dk ** -0.5, cap)
+    assert ((got - ref).abs() <= ref.abs() * 1.01 * 2 ** -8 + mag * (30 * 2 ** -11 if cap else 2 ** -8) + 2e-4).all()
+    with pytest.raises(RuntimeError, match="16 bytes"):
+        B.kv_write(q[:, :Hk, :dk].contiguous(), torch.zeros(meta.num_tokens, Hk, dv, dtype=torch.bfloat16, device="cuda"), at_odd(kpool), vpool,
+                   meta.slot_mapping)
