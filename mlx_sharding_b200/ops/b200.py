@@ -200,7 +200,7 @@ def paged_attention(q, kpool, vpool, meta: BatchMeta, scale: float, softcap: flo
     several streams at once; captured calls share one set of them, so graphs that hold some are replayed one at a time."""
     c = C()
     softcap = float(softcap or 0.0)
-    if meta.max_q_len > 1 and c.flash_prefill_takes(q, kpool, vpool, softcap, int(meta.num_seqs), int(meta.max_ctx_len)):
+    if meta.max_q_len > 1 and c.flash_prefill_takes(q, kpool, vpool, softcap, int(meta.num_seqs), int(meta.max_ctx_len), float(scale)):
         # prefill chunk / mixed batch: tensor-core causal flash attention over the paged cache
         return c.flash_prefill(q, kpool, vpool, meta.block_tables, meta.cu_seqlens, meta.context_lens, float(scale),
                                int(meta.num_tokens), softcap, int(meta.max_ctx_len))

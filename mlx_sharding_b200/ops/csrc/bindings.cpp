@@ -516,8 +516,10 @@ bool flash_short(int64_t max_ctx, int64_t tokens, int64_t seqs, int64_t heads) {
   return max_ctx > 0 && max_ctx < 128 && (tokens / 64 + seqs) * heads <= 6 * sm_count();
 }
 // whether flash_prefill takes these tensors (else: paged_attention).  Capped scores of a handful of keys: the decode kernel (Gemma-2-9B heads, one prompt
-// of 16 tokens 3.8 us there, 11.9 here; 64 tokens 12.2 / 8.2; 16 prompts of 16 20.0 / 20.1).
-bool flash_prefill_takes(const Tensor& q, const Tensor& kpool, const Tensor& vpool, double softcap, int64_t num_seqs, int64_t max_ctx) {
+// of 16 tokens 3.8 us there, 11.9 here; 64 tokens 12.2 / 8.2; 16 prompts of 16 20.0 / 20.1).  Both forms keep the maximum of the raw scores, so a score
+// factor that is not positive goes to the decode kernel, which scales first; so does a negative cap (none, there).
+bool flash_prefill_takes(const Tensor& q, const Tensor& kpool, const Tensor& vpool, double softcap, int64_t num_seqs, int64_t max_ctx, double scale) {
+  if (!(scale > 0.0) || softcap < 0.0) return false;
   if (q.dim() != 3 || q.stride(2) != 1 || kpool.dim() != 4 || vpool.dim() != 4 || q.size(2) != kpool.size(3)) return false;
   b200::FlashPrefillArgs a = flash_args(q, kpool, vpool, softcap);
   a.num_seqs = (int)num_seqs;
@@ -1689,7 +1691,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flash_prefill", &flash_prefill, py::arg("q"), py::arg("kpool"), py::arg("vpool"), py::arg("block_tables"), py::arg("cu_seqlens"),
         py::arg("context_lens"), py::arg("scale"), py::arg("num_tokens"), py::arg("softcap") = 0.0, py::arg("max_ctx") = 0,
         py::arg("wait_spins") = (int64_t)b200::kWaitSpins);
-  m.def("flash_prefill_takes", &flash_prefill_takes);
+  m.def("flash_prefill_takes", &flash_prefill_takes, py::arg("q"), py::arg("kpool"), py::arg("vpool"), py::arg("softcap"), py::arg("num_seqs"),
+        py::arg("max_ctx"), py::arg("scale") = 1.0);
   m.def("mla_prefill_prologue", &mla_prefill_prologue);
   m.def("flash_mla", &flash_mla);
   m.def("flash_mla_supported", [](int64_t num_seqs) { return b200::flash_mla_supported((int)num_seqs); });

@@ -242,3 +242,15 @@ def test_pools_at_odd_offsets(B, H, Hk, dk, dv, cap, q_lens, ctx0):
     with pytest.raises(RuntimeError, match="16 bytes"):
         B.kv_write(q[:, :Hk, :dk].contiguous(), torch.zeros(meta.num_tokens, Hk, dv, dtype=torch.bfloat16, device="cuda"), at_odd(kpool), vpool,
                    meta.slot_mapping)
+
+
+@pytest.mark.parametrize("H,Hk,dk,dv", [(4, 2, 256, 256), (8, 2, 128, 128)])
+@pytest.mark.parametrize("factor,cap", [(-1.0, 0.0), (0.0, 0.0), (-1.0, 30.0), (1.0, -1.0)])
+def test_prompts_with_any_score_factor(B, H, Hk, dk, dv, factor, cap):
+    """A factor that is not positive turns the order of the scores around; a negative cap is none."""
+    q_lens, ctx0 = [150, 40], [0, 70]
+    meta, tables, kpool, vpool, rnd = paged(q_lens, ctx0, Hk, dk, dv, 64)
+    q, scale = rnd(meta.num_tokens, H, dk) * 2, factor * dk ** -0.5
+    got = B.paged_attention(q, kpool, vpool, meta, scale, cap).double()
+    ref, mag = exact(q, kpool, vpool, tables, q_lens, ctx0, scale, max(cap, 0.0))
+    assert ((got - ref).abs() <= ref.abs() * 1.01 * 2 ** -8 + mag * (30 * 2 ** -11 if cap > 0 else 2 ** -16) + 2e-4).all()
