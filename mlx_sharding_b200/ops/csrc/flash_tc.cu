@@ -16,12 +16,15 @@
 //   * S is double buffered, the scores of each stream and the second products have an issuing thread of their own (issuing, not the tensor pipe, was
 //     what one thread for all was bound by: ~100 cycles per product), so scores run a tile ahead of the softmax warps; P overwrites its own score buffer.  A buffer is written again only after the product that reads
 //     it has completed (its commit is waited for);
-//   * one thread per row: no shuffles; the running maximum is allowed to lag by 2^8 before the accumulator in TMEM is rescaled (p <= 256 stays
-//     exact in fp32 sums and has the same relative error as bf16), so rescales are rare after the first tiles;
+//   * one thread per row: no shuffles; the running maximum may lag by 2^8 before the accumulator in TMEM is rescaled, so rescales are rare after
+//     the first tiles;
+//   * probabilities enter the second product as two bf16 terms (error 2^-17 of each, where a lagging maximum leaves no probability exact; a visible
+//     infinity in V gives NaN, as the low term may be 0 or of the other sign).  One term costs half of the second product's tensor time, but with the lag
+//     its error alone is above the result's rounding: error of the op against 64 bits at scores with a spread of 2: mma.sync form (maximum exact, one
+//     term) 1.838e-3, one term and the lag 2.104e-3, one term and no lag 1.838e-3, two terms and the lag 1.647e-3.  B200, Llama-3-8B heads 2 x 2 k / 1 x
+//     8 k tokens, DeepSeek-V2-Lite 2 k behind 6 k: 101 / 475 / 143 us, 122 / 577 / 176 without the lag, 106 / 565 / 166 with two terms;
 //   * heads of 256 (Gemma-2): the accumulator takes 256 columns, so there is one stream, whose rows' 64 scores are shared by two threads, and
 //     three score buffers;
-//   * kSplitP: probabilities enter the second product as two bf16 terms (error 2^-16), for the paths that held them in fp32, and for SINK, where the
-//     lagging maximum would otherwise cost the dominant key's exactness (error against 64 bits 0.0022 instead of 0.0019);
 //   * MLA: the decompressed keys / values are read where the kv_b product left them ([rows, heads * (nope + v)]), the shared rotary key from
 //     the latent pool's pages: no per-head K / V pool is assembled.
 //   * SINK (windowed attention of the hybrid stacks, sinkattn.cu): only tiles with visible keys are walked; the fp32 queries enter the first product
@@ -50,7 +53,7 @@ constexpr float kLazy = 8.f;                  // how far (log2) the maximum may 
 
 constexpr int kMaxSeqs = 512;                 // sequences of a step that the item table holds
 
-enum : int { kMla = 1, kCap = 2, kSplitP = 4, kSink = 8 };
+enum : int { kMla = 1, kCap = 2, kSink = 4 };
 
 struct FlashTcParams {
   const int* block_tables; int max_blocks;
@@ -176,7 +179,7 @@ template <int DK, int DV, int MODE>
 __global__ void __launch_bounds__(kFlashThreads, 1)
 flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                 const __grid_constant__ CUtensorMap tmap_pe, const FlashTcParams p) {
-  constexpr bool MLA = (MODE & kMla) != 0, CAP = (MODE & kCap) != 0, PSPLIT = (MODE & kSplitP) != 0, SINK = (MODE & kSink) != 0;
+  constexpr bool MLA = (MODE & kMla) != 0, CAP = (MODE & kCap) != 0, SINK = (MODE & kSink) != 0;
   constexpr int NS = ft_streams(DV), NB = ft_bufs(DV), ST = ft_stages(DK, DV, MODE);
   constexpr int CK = DK / 64, CV = DV / 64;
   constexpr int QB = ft_q_bytes(DK, MODE), KB = kKeys * DK * 2, VB = kKeys * DV * 2, CHUNK = kKeys * 128;
@@ -421,7 +424,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             for (int ks = 0; ks < kKeys / 16; ++ks) {
               const uint64_t bd = ft_desc_mn(va + ks * 2048, CHUNK, 1024);
               umma_f16_ts(d, pa + 8 * ks, bd, IDESC_O, (j | ks) ? 1u : 0u);
-              if constexpr (PSPLIT) umma_f16_ts(d, pa + 32 + 8 * ks, bd, IDESC_O, 1u);
+              umma_f16_ts(d, pa + 32 + 8 * ks, bd, IDESC_O, 1u);
             }
             umma_commit(&o_done[s * NB + g[s] % NB]);
             ++g[s];
@@ -542,20 +545,20 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         const float sub = m == -INFINITY ? 0.f : -m;
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t hi[PAIRS], lo[PSPLIT ? PAIRS : 1];
+        uint32_t hi[PAIRS], lo[PAIRS];
 #pragma unroll
         for (int c = 0; c < PAIRS; ++c) {
           const float a = exp2f(fmaf(x[2 * c], sl2, sub)), b = exp2f(fmaf(x[2 * c + 1], sl2, sub));
           sum[c & 3] += a + b;
           hi[c] = pack_bf16(a, b);
-          if constexpr (PSPLIT) lo[c] = pack_bf16(a - bf16_lo(hi[c]), b - bf16_hi(hi[c]));
+          lo[c] = pack_bf16(a - bf16_lo(hi[c]), b - bf16_hi(hi[c]));
         }
         l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
         if constexpr (NS == 1) named_bar_sync(2, 256);                           // P overwrites the scores: both halves of a row have been read
 #pragma unroll
         for (int c = 0; c < PAIRS; c += 16) {
           tmem_st16(buf + half * PAIRS + c, hi + c);
-          if constexpr (PSPLIT) tmem_st16(buf + 32 + half * PAIRS + c, lo + c);
+          tmem_st16(buf + 32 + half * PAIRS + c, lo + c);
         }
         tmem_st_wait();
         const int vend = v_end - tile0;
@@ -715,13 +718,13 @@ cudaError_t flash_tc_launch(const FlashPrefillArgs& a, cudaStream_t s) {
   if (!ft_map_q(&tq, a.q, a.dk_, a.q_heads, a.tokens, a.q_ld_h, a.q_ld_t) || !ft_map_2d(&tk, a.kpool, a.dk_, a.pool_rows, a.dk_, p.box_rows) ||
       !ft_map_2d(&tv, a.vpool, a.dv_, a.pool_rows, a.dv_, p.box_rows))
     return cudaErrorInvalidValue;
-  if (a.softcap > 0.f) {                       // the capped path held its probabilities in fp32
-    if (a.dk_ == 256) return launch_flash_tc<256, 256, kCap | kSplitP>(tq, tk, tv, tk, p, a.tokens, s);
-    if (a.dk_ == 192) return launch_flash_tc<192, 128, kCap | kSplitP>(tq, tk, tv, tk, p, a.tokens, s);
-    if (a.dk_ == 128) return launch_flash_tc<128, 128, kCap | kSplitP>(tq, tk, tv, tk, p, a.tokens, s);
-    return launch_flash_tc<64, 64, kCap | kSplitP>(tq, tk, tv, tk, p, a.tokens, s);
+  if (a.softcap > 0.f) {
+    if (a.dk_ == 256) return launch_flash_tc<256, 256, kCap>(tq, tk, tv, tk, p, a.tokens, s);
+    if (a.dk_ == 192) return launch_flash_tc<192, 128, kCap>(tq, tk, tv, tk, p, a.tokens, s);
+    if (a.dk_ == 128) return launch_flash_tc<128, 128, kCap>(tq, tk, tv, tk, p, a.tokens, s);
+    return launch_flash_tc<64, 64, kCap>(tq, tk, tv, tk, p, a.tokens, s);
   }
-  if (a.dk_ == 256) return launch_flash_tc<256, 256, kSplitP>(tq, tk, tv, tk, p, a.tokens, s);
+  if (a.dk_ == 256) return launch_flash_tc<256, 256, 0>(tq, tk, tv, tk, p, a.tokens, s);
   if (a.dk_ == 192) return launch_flash_tc<192, 128, 0>(tq, tk, tv, tk, p, a.tokens, s);
   if (a.dk_ == 128) return launch_flash_tc<128, 128, 0>(tq, tk, tv, tk, p, a.tokens, s);
   return launch_flash_tc<64, 64, 0>(tq, tk, tv, tk, p, a.tokens, s);
@@ -762,8 +765,8 @@ cudaError_t flash_sink_launch(const SinkAttnArgs& a, const int* context_lens, lo
   p.block = a.block; p.window = a.window; p.keep = a.keep; p.out_mult = a.out_mult;
   CUtensorMap tk, tv;
   if (!ft_map_2d(&tk, a.kpool, a.D, pool_rows, a.D, p.box_rows) || !ft_map_2d(&tv, a.vpool, a.V, pool_rows, a.V, p.box_rows)) return cudaErrorInvalidValue;
-  if (a.D == 128) return launch_flash_tc<128, 128, kSink | kSplitP>(tk, tk, tv, tk, p, tokens, s);
-  return launch_flash_tc<64, 64, kSink | kSplitP>(tk, tk, tv, tk, p, tokens, s);
+  if (a.D == 128) return launch_flash_tc<128, 128, kSink>(tk, tk, tv, tk, p, tokens, s);
+  return launch_flash_tc<64, 64, kSink>(tk, tk, tv, tk, p, tokens, s);
 }
 
 }  // namespace b200

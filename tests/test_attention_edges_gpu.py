@@ -254,3 +254,20 @@ def test_prompts_with_any_score_factor(B, H, Hk, dk, dv, factor, cap):
     got = B.paged_attention(q, kpool, vpool, meta, scale, cap).double()
     ref, mag = exact(q, kpool, vpool, tables, q_lens, ctx0, scale, max(cap, 0.0))
     assert ((got - ref).abs() <= ref.abs() * 1.01 * 2 ** -8 + mag * (30 * 2 ** -11 if cap > 0 else 2 ** -16) + 2e-4).all()
+
+
+@pytest.mark.parametrize("H,Hk,dk,dv,cap", [(8, 2, 128, 128, 0.0), (4, 4, 192, 128, 0.0), (4, 2, 64, 64, 0.0), (4, 2, 256, 256, 0.0), (4, 2, 128, 128, 1e4)])
+@pytest.mark.parametrize("gain", [0.5, 2.0, 6.0])
+def test_prompt_probabilities_cost_nothing(B, H, Hk, dk, dv, cap, gain):
+    """Flat to peaked softmaxes, maxima that grow by less than the lag: beside the rounding of the result to bf16 there is the 2^-17 of a probability in two
+    terms, with fp32 sums.  (One term of 2^-9 would add a quarter to the whole error.)  A cap far above the scores changes them by less than 2^-11."""
+    q_lens, ctx0 = [400, 129], [0, 900]
+    meta, tables, kpool, vpool, rnd = paged(q_lens, ctx0, Hk, dk, dv, 64)
+    q = rnd(meta.num_tokens, H, dk) * gain
+    got = B.paged_attention(q, kpool, vpool, meta, dk ** -0.5, cap).double()
+    ref, mag = exact(q, kpool, vpool, tables, q_lens, ctx0, dk ** -0.5, cap)
+    rounding = (ref.to(torch.bfloat16).double() - ref).norm()
+    if cap:
+        assert (got - ref).norm() <= 1.02 * rounding + mag.norm() * 4 * gain * 2 ** -11
+    else:
+        assert (got - ref).norm() <= 1.02 * rounding + mag.norm() * 2 ** -16
