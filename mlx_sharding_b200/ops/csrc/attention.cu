@@ -258,6 +258,121 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, long long q_ld_t, long 
   }
 }
 
+// Contexts of a few keys with one or two query heads per kv head: of the products above at most an eighth is useful, and a tile is always 16 keys.  Here lanes
+// split the head dimension, a warp takes four keys at a time in registers, products are finished with shuffles, and nothing goes through shared memory
+// but the merge of the four warps.  One split.
+constexpr int kVecKeys = 4;
+template <int DK, int DV, int G>
+__global__ void __launch_bounds__(128)
+paged_vector_kernel(const __nv_bfloat16* __restrict__ q, long long q_ld_t, long long q_ld_h, const __nv_bfloat16* __restrict__ kpool,
+                    const __nv_bfloat16* __restrict__ vpool, const int* __restrict__ block_tables, int max_blocks, const int* __restrict__ positions,
+                    const int* __restrict__ token_seq, int kv_heads, int page, float scale, float softcap, __nv_bfloat16* __restrict__ out, long long o_ld_t) {
+  pdl_sync();  // PDL: predecessor's writes visible; let the successor start its prologue
+  constexpr int PK = DK / 64, PV = DV / 64, WARPS = 4;          // bf16 pairs of a row that a lane holds
+  const int t = blockIdx.x, hk = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kv_len = positions[t] + 1;
+  const int* bt = block_tables + (size_t)token_seq[t] * max_blocks;
+  float qf[G][2 * PK], m[G], l[G], acc[G][2 * PV];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const __nv_bfloat16* qp = q + (size_t)t * q_ld_t + (size_t)(hk * G + g) * q_ld_h;
+#pragma unroll
+    for (int i = 0; i < PK; ++i) {
+      const uint32_t u = reinterpret_cast<const uint32_t*>(qp)[lane + 32 * i];
+      qf[g][2 * i] = bf16_lo(u) * scale;
+      qf[g][2 * i + 1] = bf16_hi(u) * scale;
+    }
+    m[g] = -INFINITY; l[g] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2 * PV; ++i) acc[g][i] = 0.f;
+  }
+  for (int base = warp * kVecKeys; base < kv_len; base += WARPS * kVecKeys) {
+    uint32_t kreg[kVecKeys][PK], vreg[kVecKeys][PV];
+#pragma unroll
+    for (int j = 0; j < kVecKeys; ++j) {
+      const int pos = min(base + j, kv_len - 1);                // behind the end: the last key, left out below
+      const size_t row = ((size_t)bt[pos / page] * kv_heads + hk) * page + pos % page;
+      const uint32_t* kp = reinterpret_cast<const uint32_t*>(kpool + row * DK);
+      const uint32_t* vp = reinterpret_cast<const uint32_t*>(vpool + row * DV);
+#pragma unroll
+      for (int i = 0; i < PK; ++i) kreg[j][i] = kp[lane + 32 * i];
+#pragma unroll
+      for (int i = 0; i < PV; ++i) vreg[j][i] = vp[lane + 32 * i];
+    }
+#pragma unroll
+    for (int j = 0; j < kVecKeys; ++j) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < PK; ++i) {
+          s += qf[g][2 * i] * bf16_lo(kreg[j][i]);
+          s += qf[g][2 * i + 1] * bf16_hi(kreg[j][i]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+        if (base + j < kv_len) {
+          const float mn = fmaxf(m[g], s), corr = __expf(m[g] - mn), p = __expf(s - mn);
+          l[g] = l[g] * corr + p;
+#pragma unroll
+          for (int i = 0; i < PV; ++i) {
+            acc[g][2 * i] = acc[g][2 * i] * corr + p * bf16_lo(vreg[j][i]);
+            acc[g][2 * i + 1] = acc[g][2 * i + 1] * corr + p * bf16_hi(vreg[j][i]);
+          }
+          m[g] = mn;
+        }
+      }
+    }
+  }
+  __shared__ float s_m[WARPS][G], s_l[WARPS][G], s_acc[WARPS][G][DV];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    if (lane == 0) { s_m[warp][g] = m[g]; s_l[warp][g] = l[g]; }
+#pragma unroll
+    for (int i = 0; i < PV; ++i) {
+      s_acc[warp][g][2 * (lane + 32 * i)] = acc[g][2 * i];
+      s_acc[warp][g][2 * (lane + 32 * i) + 1] = acc[g][2 * i + 1];
+    }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < G * DV; idx += 128) {
+    const int g = idx / DV, d = idx % DV;
+    float mm = -INFINITY, ll = 0.f, a = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, s_m[w][g]);
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float c = s_m[w][g] == -INFINITY ? 0.f : __expf(s_m[w][g] - mm);
+      ll += s_l[w][g] * c;
+      a += s_acc[w][g][d] * c;
+    }
+    out[(size_t)t * o_ld_t + (size_t)(hk * G + g) * DV + d] = __float2bfloat16_rn(ll > 0.f ? a / ll : 0.f);
+  }
+}
+
+template <int DK, int DV, int G>
+cudaError_t launch_vector(const PagedAttnArgs& a, cudaStream_t s) {
+  (void)launch_pdl(paged_vector_kernel<DK, DV, G>, dim3(a.T, a.kv_heads), dim3(128), 0, s, static_cast<const __nv_bfloat16*>(a.q), a.q_ld_t, a.q_ld_h,
+                   static_cast<const __nv_bfloat16*>(a.kpool), static_cast<const __nv_bfloat16*>(a.vpool), a.block_tables, a.max_blocks, a.positions,
+                   a.token_seq, a.kv_heads, a.page, a.scale, a.softcap, static_cast<__nv_bfloat16*>(a.out), a.o_ld_t);
+  return cudaGetLastError();
+}
+
+// Where the vector form is faster.  B200, us, vector / matrix form, by the bound of the contexts: one query head per kv head, 16 heads of 192 / 128, 1 token
+// 2.2 / 2.7 (up to 16 keys; 17: 3.2 / 2.7), 8 tokens 2.4 / 2.8 (16; 17: 3.3 / 3.2), 64 tokens 3.0 / 3.7 (1), 3.9 / 3.8 (8), 5.1 / 3.8 (16), 256 tokens 8.5 / 11.1 (8), 11.7 / 11.1 (16),
+// 1024 tokens 42.8 / 45.7 (16), 54.2 / 53.6 (17); 32 heads of 128, 1 token 2.3 / 2.5 (16), 8 tokens 2.5 / 2.7 (8), 2.8 / 2.6 (16), 64 tokens 4.9 / 5.0 (8), 256 tokens 14.1 / 12.9 (8);
+// 16 heads of 256, 8 tokens 2.6 / 3.0 (16), 64 tokens 3.8 / 4.5 (8), 5.2 / 4.5 (16), 6.0 / 7.5 (17), 8.0 / 7.5 (32), 1024 tokens 71 / 77 (17), 96 / 90 (32); two query heads
+// per kv head, 8 of 256, 64 tokens 4.3 / 4.5 (8), 5.0 / 4.5 (16), 256 tokens 10.6 / 8.4 (8).  Heads of 64 and larger groups: the matrix form is as fast or faster from one key on.
+bool vector_form(int dk, int G, int max_ctx, long long pairs) {
+  if (max_ctx <= 0 || max_ctx > 24) return false;
+  if (G == 2 && dk == 256) return max_ctx <= 8 && pairs <= 512;
+  if (G != 1 || dk < 128) return false;
+  if (max_ctx <= 8) return dk > 128 || pairs <= 2048;
+  if (max_ctx <= 16) return pairs <= (dk > 128 ? 128 : 32) || (dk == 192 && pairs >= 8192);
+  return dk == 256 && pairs >= 1024;
+}
+
 template <int DK, int DV, int WARPS, int STAGES>
 cudaError_t launch_decode_ring(const PagedAttnArgs& a, cudaStream_t s) {
   constexpr int smem = dec_smem(DK, DV, WARPS, STAGES);
@@ -312,6 +427,11 @@ cudaError_t paged_attention_launch(const PagedAttnArgs& a, cudaStream_t s) {
   if (a.nsplit > 1 && (a.part_acc == nullptr || a.part_ml == nullptr || a.tickets == nullptr)) return cudaErrorInvalidValue;
   const int G = a.q_heads / a.kv_heads;
   const bool pow2 = G == 1 || G == 2 || G == 4 || G == 8;
+  if (a.nsplit == 1 && a.q_heads == G * a.kv_heads && vector_form(a.dk_, G, a.max_ctx, (long long)a.T * a.kv_heads)) {
+    if (a.dk_ == 192 && a.dv_ == 128) return launch_vector<192, 128, 1>(a, s);
+    if (a.dk_ == 128 && a.dv_ == 128) return launch_vector<128, 128, 1>(a, s);
+    if (a.dk_ == 256 && a.dv_ == 256) return G == 1 ? launch_vector<256, 256, 1>(a, s) : launch_vector<256, 256, 2>(a, s);
+  }
   if (a.dk_ == 192 && a.dv_ == 128 && G == 1) return launch_decode<192, 128>(a, s);       // DeepSeek-V2 MLA, decompressed cache
   if (a.dk_ == 128 && a.dv_ == 128 && pow2) return launch_decode<128, 128>(a, s);         // Llama-3-8B: 32 q heads / 8 kv heads
   if (a.dk_ == 256 && a.dv_ == 256 && pow2 && G <= 2) return launch_decode<256, 256>(a, s);   // Gemma-2-9B

@@ -271,3 +271,15 @@ def test_prompt_probabilities_cost_nothing(B, H, Hk, dk, dv, cap, gain):
         assert (got - ref).norm() <= 1.02 * rounding + mag.norm() * 4 * gain * 2 ** -11
     else:
         assert (got - ref).norm() <= 1.02 * rounding + mag.norm() * 2 ** -16
+
+
+# one or two query heads per kv head over a few keys: both sides of the lines between the vector and the matrix form, in keys and in rows
+@pytest.mark.parametrize("H,Hk,dk,dv,cap", [(16, 16, 192, 128, 0.0), (32, 32, 128, 128, 0.0), (4, 4, 256, 256, 0.0), (16, 8, 256, 256, 50.0)])
+@pytest.mark.parametrize("n,keys", [(1, 1), (3, 8), (3, 9), (2, 16), (9, 16), (600, 16), (2, 17), (300, 24), (5, 25), (70, 8), (65, 7)])
+def test_paged_decode_few_keys(B, H, Hk, dk, dv, cap, n, keys):
+    ctx = [keys - 1] + [i * 5 % keys for i in range(n - 1)]
+    meta, tables, kpool, vpool, rnd = paged([1] * n, ctx, Hk, dk, dv, 16)
+    q = rnd(n, H, dk) * 2
+    got = B.paged_attention(q, kpool, vpool, meta, dk ** -0.5, cap).double()
+    ref, mag = exact(q, kpool, vpool, tables, [1] * n, ctx, dk ** -0.5, cap)
+    assert ((got - ref).abs() <= ref.abs() * 2 ** -8 + mag * (30 * 2 ** -11 if cap else 0.0) + 2e-4).all(), float((got - ref).abs().max())
