@@ -27,24 +27,7 @@ namespace {
 
 constexpr int kBM = 64, kBN = 64, kWarps = 4, kThreads = 128;
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem)));
-}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) { mma_m16n8k16(d, a[0], a[1], a[2], a[3], b0, b1); }
 
 struct SinkForm {                            // what the SINK form adds (unused otherwise)
   const float* q32;                          // [T, heads, d]
@@ -53,10 +36,6 @@ struct SinkForm {                            // what the SINK form adds (unused 
   int d, v, block, window, keep;
   float scale, out_mult;                     // scale multiplies the queries (scale_log2 is log2(e) alone)
 };
-
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem)));
-}
 
 template <int DK, int DV, bool SINK, int DIST = 0>
 __global__ void __launch_bounds__(kThreads)
@@ -119,10 +98,10 @@ flash_prefill_kernel(const __nv_bfloat16* __restrict__ q, long long q_ld_t, long
     const __nv_bfloat16* gV = vpool + row * V;
 #pragma unroll
     for (int c = 0; c < DK / 16; ++c)
-      if (!SINK || 2 * c + lc < KC) cp_async16(dK + (2 * c + lc) * 8, gK + (2 * c + lc) * 8);
+      if (!SINK || 2 * c + lc < KC) cp_async16(smem_u32(dK + (2 * c + lc) * 8), gK + (2 * c + lc) * 8);
 #pragma unroll
     for (int c = 0; c < DV / 16; ++c)
-      if (!SINK || 2 * c + lc < VC) cp_async16(dV + (2 * c + lc) * 8, gV + (2 * c + lc) * 8);
+      if (!SINK || 2 * c + lc < VC) cp_async16(smem_u32(dV + (2 * c + lc) * 8), gV + (2 * c + lc) * 8);
     cp_async_commit();
   };
 
@@ -202,7 +181,7 @@ flash_prefill_kernel(const __nv_bfloat16* __restrict__ q, long long q_ld_t, long
 #pragma unroll
         for (int nt = 0; nt < kBN / 8; nt += 2) {
           uint32_t kb[4];
-          ldmatrix_x4(kb, kr + nt * 8 * KS + ks * 16);
+          ldmatrix_x4(kb, smem_u32(kr + nt * 8 * KS + ks * 16));
           mma_bf16(s[nt], qa[ks], kb[0], kb[1]);
           mma_bf16(s[nt + 1], qa[ks], kb[2], kb[3]);
           if constexpr (SINK) {
@@ -273,7 +252,7 @@ flash_prefill_kernel(const __nv_bfloat16* __restrict__ q, long long q_ld_t, long
       for (int nt2 = 0; nt2 < DV / 16; ++nt2) {
         uint32_t vb[4];
         // lanes 0-15: rows kk*16 + (lane & 15) at column nt2*16; lanes 16-31: same rows at column +8
-        ldmatrix_x4_trans(vb, tV + (kk * 16 + (lane & 15)) * VS + nt2 * 16 + ((lane >> 4) << 3));
+        ldmatrix_x4_trans(vb, smem_u32(tV + (kk * 16 + (lane & 15)) * VS + nt2 * 16 + ((lane >> 4) << 3)));
         mma_bf16(o[nt2 * 2], pa[kk], vb[0], vb[1]);
         mma_bf16(o[nt2 * 2 + 1], pa[kk], vb[2], vb[3]);
       }

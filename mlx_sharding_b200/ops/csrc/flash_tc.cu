@@ -36,6 +36,7 @@
 // decode kernel (2 x 1 k tokens of Gemma-2-9B 1853 us, here 53 us).
 #include <cuda.h>
 
+#include "gemm_tmap.h"
 #include "kernels.h"
 #include "launch.h"
 #include "ptx.cuh"
@@ -81,19 +82,10 @@ __host__ __device__ constexpr int ft_smem(int dk, int dv, int mode) {
 __host__ __device__ constexpr uint32_t ft_idesc(uint32_t M, uint32_t N, uint32_t b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
-// MN-major, 128B-swizzled operand: 64 MN-elements are one 128 B line, K rows 128 B apart, groups of 8 K rows `sbo`, 64-element MN blocks `lbo` apart
-B200_DEVICE uint64_t ft_desc_mn(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  return static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4) | static_cast<uint64_t>(lbo >> 4) << 16 | static_cast<uint64_t>(sbo >> 4) << 32 |
-         static_cast<uint64_t>(1) << 46 | static_cast<uint64_t>(2) << 61;
-}
 // A operand from TMEM (row = lane, two bf16 per 32-bit column), B from shared memory
 B200_DEVICE void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-B200_DEVICE void ft_tma_3d(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 B200_DEVICE void ft_tma_2d(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -318,7 +310,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             alive = alive && wait(&q_empty[s], (qn[s] & 1) ^ 1);
             if (!alive) continue;
             mbar_arrive_expect_tx(&q_full[s], QB);
-            for (int c = 0; c < CK; ++c) ft_tma_3d(smem_u32(q_smem + s * QB + c * kRows * 128), &tmap_q, &q_full[s], c * 64, it.head[s], it.tok[s]);
+            for (int c = 0; c < CK; ++c) tma_load_3d(q_smem + s * QB + c * kRows * 128, &tmap_q, &q_full[s], c * 64, it.head[s], it.tok[s]);
             ++qn[s];
           }
         }
@@ -422,7 +414,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             const uint32_t va = smem_u32(v_smem + (kv % ST) * VB), pa = tmem_base + (s * NB + g[s] % NB) * 64, d = tmem_base + O_COL + s * DV;
 #pragma unroll
             for (int ks = 0; ks < kKeys / 16; ++ks) {
-              const uint64_t bd = ft_desc_mn(va + ks * 2048, CHUNK, 1024);
+              const uint64_t bd = umma_desc_mn_sw128(va + ks * 2048, CHUNK, 1024);
               umma_f16_ts(d, pa + 8 * ks, bd, IDESC_O, (j | ks) ? 1u : 0u);
               umma_f16_ts(d, pa + 32 + 8 * ks, bd, IDESC_O, 1u);
             }
@@ -650,28 +642,16 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn ft_encode() {
-  static EncodeTiledFn fn = [] {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess) ptr = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(ptr);
-  }();
-  return fn;
-}
 bool ft_map_2d(CUtensorMap* m, const void* ptr, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_rows) {
   const cuuint64_t dims[2] = {cols, rows}, strides[1] = {ld * 2};
   const cuuint32_t box[2] = {64, box_rows}, one[2] = {1, 1};
-  return ft_encode()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return tensor_map_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 bool ft_map_q(CUtensorMap* m, const void* ptr, uint64_t dk, uint64_t heads, uint64_t tokens, uint64_t ld_h, uint64_t ld_t) {
   const cuuint64_t dims[3] = {dk, heads, tokens}, strides[2] = {ld_h * 2, ld_t * 2};
   const cuuint32_t box[3] = {64, 1, kRows}, one[3] = {1, 1, 1};
-  return ft_encode()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return tensor_map_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -703,7 +683,7 @@ bool ft_pages(int page) { return page % kKeys == 0 || page == 16 || page == 32; 
 bool flash_tc_supported(const FlashPrefillArgs& a) {
   const bool dims = (a.dk_ == 128 && a.dv_ == 128) || (a.dk_ == 192 && a.dv_ == 128) || (a.dk_ == 64 && a.dv_ == 64) || (a.dk_ == 256 && a.dv_ == 256);
   return dims && ft_pages(a.page) && a.q_heads % a.kv_heads == 0 && a.q_ld_t % 8 == 0 && a.q_ld_h % 8 == 0 && ft_aligned(a.q) && ft_aligned(a.kpool) &&
-         ft_aligned(a.vpool) && ft_aligned(a.out) && a.o_ld_t % 8 == 0 && a.num_seqs <= kMaxSeqs && a.pool_rows < (1LL << 31) && ft_encode() != nullptr;
+         ft_aligned(a.vpool) && ft_aligned(a.out) && a.o_ld_t % 8 == 0 && a.num_seqs <= kMaxSeqs && a.pool_rows < (1LL << 31) && tensor_map_encoder() != nullptr;
 }
 
 cudaError_t flash_tc_launch(const FlashPrefillArgs& a, cudaStream_t s) {
@@ -735,7 +715,7 @@ bool flash_mla_supported(int num_seqs) { return num_seqs <= kMaxSeqs; }
 cudaError_t flash_mla_launch(const FlashMlaArgs& a, cudaStream_t s) {
   if (a.num_seqs == 0 || a.tokens == 0) return cudaSuccess;
   if (a.page % kKeys != 0 || a.q_ld_t % 8 != 0 || a.q_ld_h % 8 != 0 || a.kv_ld % 8 != 0 || !ft_aligned(a.q) || !ft_aligned(a.kv) || !ft_aligned(a.pool) ||
-      !ft_aligned(a.out) || a.o_ld_t % 8 != 0 || a.kv_rows >= (1LL << 31) || a.pool_rows >= (1LL << 31) || a.num_seqs > kMaxSeqs || ft_encode() == nullptr)
+      !ft_aligned(a.out) || a.o_ld_t % 8 != 0 || a.kv_rows >= (1LL << 31) || a.pool_rows >= (1LL << 31) || a.num_seqs > kMaxSeqs || tensor_map_encoder() == nullptr)
     return cudaErrorInvalidValue;
   FlashTcParams p = {};
   p.block_tables = a.block_tables; p.max_blocks = a.max_blocks; p.cu_seqlens = a.cu_seqlens; p.context_lens = a.context_lens; p.num_seqs = a.num_seqs;
@@ -751,7 +731,7 @@ cudaError_t flash_mla_launch(const FlashMlaArgs& a, cudaStream_t s) {
 bool flash_sink_takes(const SinkAttnArgs& a, long long pool_rows) {
   const bool dims = (a.D == 128 && a.V == 128) || (a.D == 64 && a.V == 64);
   return dims && a.slopes == nullptr && a.bias == nullptr && ft_pages(a.page) && a.H % a.G == 0 && a.B > 0 && a.B <= kMaxSeqs && ft_aligned(a.q) &&
-         ft_aligned(a.kpool) && ft_aligned(a.vpool) && ft_aligned(a.out) && a.ld_out % 8 == 0 && pool_rows < (1LL << 31) && ft_encode() != nullptr;
+         ft_aligned(a.kpool) && ft_aligned(a.vpool) && ft_aligned(a.out) && a.ld_out % 8 == 0 && pool_rows < (1LL << 31) && tensor_map_encoder() != nullptr;
 }
 
 cudaError_t flash_sink_launch(const SinkAttnArgs& a, const int* context_lens, long long pool_rows, int tokens, const WaitBound& wait, cudaStream_t s) {

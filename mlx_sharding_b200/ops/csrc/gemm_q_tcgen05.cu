@@ -14,6 +14,7 @@
 #include <unordered_map>
 
 #include "gemm_q_common.cuh"
+#include "gemm_tmap.h"
 #include "launch.h"
 
 namespace b200 {
@@ -200,22 +201,6 @@ gemm_swapab_q_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_c
 // ================================================================================================ host side
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn q_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      return nullptr;
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
 struct QKey {
   const void* ptr; uint64_t d0, d1, ld; uint32_t b0, b1; int kind;
   bool operator==(const QKey& o) const { return ptr == o.ptr && d0 == o.d0 && d1 == o.d1 && ld == o.ld && b0 == o.b0 && b1 == o.b1 && kind == o.kind; }
@@ -237,7 +222,7 @@ bool q_make_tmap(CUtensorMap* m, int kind, const void* ptr, uint64_t d0, uint64_
   std::lock_guard<std::mutex> lock(g_qmutex);
   auto it = g_qcache.find(key);
   if (it != g_qcache.end()) { *m = it->second; return true; }
-  EncodeTiledFn fn = q_encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (fn == nullptr) return false;
   const uint32_t esz = kind == 1 ? 4 : 2;
   cuuint64_t dims[2] = {d0, d1};

@@ -193,23 +193,17 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 }
 
 // ================================================================================================ host side
-namespace {
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
+EncodeTiledFn tensor_map_encoder() {
+  static EncodeTiledFn fn = [] {
     void* ptr = nullptr;
     cudaDriverEntryPointQueryResult qres;
-    cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
-    if (e != cudaSuccess || qres != cudaDriverEntryPointSuccess || ptr == nullptr) return nullptr;
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess || qres != cudaDriverEntryPointSuccess) ptr = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(ptr);
+  }();
   return fn;
 }
+
+namespace {
 
 // Descriptor cache: encoding a tensor map costs a few microseconds of host time; weights (and the static
 // activation buffers of graph-captured steps) are encoded once.
@@ -243,7 +237,7 @@ bool make_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, ui
 }
 
 bool encode_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (fn == nullptr) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
@@ -297,7 +291,7 @@ bool gemm_make_tmap_u8(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t 
   std::lock_guard<std::mutex> lock(g_tmap_mutex);
   auto it = g_tmap_cache.find(key);
   if (it != g_tmap_cache.end()) { *m = it->second; return true; }
-  EncodeTiledFn fn = get_encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (fn == nullptr) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld};

@@ -24,6 +24,7 @@
 // Decode only (one query token per sequence); prefill chunks take the decompressing path (models/deepseek_v2.py).
 #include <cuda.h>
 
+#include "gemm_tmap.h"
 #include "kernels.h"
 #include "launch.h"
 #include "ptx.cuh"
@@ -52,25 +53,6 @@ constexpr uint32_t idesc(uint32_t M, uint32_t N, uint32_t a_mn_major) {
 }
 constexpr uint32_t kIdescQK = idesc(64, kHeads, 0);
 constexpr uint32_t kIdescPV = idesc(128, kHeads, 1);
-
-// MN-major, 128B-swizzled operand (cute canonical layout ((8,n),(8,k)):((1,LBO),(8,SBO)) in 16-byte units): 64 MN-elements are
-// contiguous (one 128 B line), 8 consecutive K rows are 128 B apart, groups of 8 K rows are SBO apart, 64-element MN blocks LBO apart.
-B200_DEVICE uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>(lbo_bytes >> 4) << 16;
-  d |= static_cast<uint64_t>(sbo_bytes >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-
-B200_DEVICE void tma_load_3d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
 
 struct MlaParams {
   const int* block_tables; int max_blocks;
@@ -448,22 +430,6 @@ mla_prologue_kernel(__nv_bfloat16* __restrict__ q, long long q_ld_t, const __nv_
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      return nullptr;
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
 }  // namespace
 
 cudaError_t mla_prologue_launch(void* q, long long q_ld_t, int q_dim, const void* ckv, long long ckv_ld_t, const void* kpe, long long pe_ld_t,
@@ -487,7 +453,7 @@ cudaError_t mla_decode_launch(const void* q, long long q_ld_t, int B, const void
                               int nsplit, float* workspace, void* out, long long o_ld_t, long long* dbg, cudaStream_t s) {
   if (B == 0) return cudaSuccess;
   if (page != kTileTok || (q_ld_t % 8) != 0) return cudaErrorInvalidValue;
-  EncodeTiledFn fn = encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (fn == nullptr) return cudaErrorUnknown;
   CUtensorMap tq, tkv;
   {
