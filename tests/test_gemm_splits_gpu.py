@@ -29,3 +29,19 @@ def test_split_reduction(T, splits, N, K):
         want = torch.nn.functional.silu(g) * u
         # the gate's sum and the fast exponential: 2^-8 relative covers both beside the rounding of the result
         assert ((got - want).abs() <= want.abs() * 2 ** -6 + mag * 2 + 1e-3).all()
+
+
+@pytest.mark.parametrize("T", [1, 8, 64, 100])
+@pytest.mark.parametrize("splits", [0, 1, 2, 4])
+def test_squared_relu_of_split_sums(T, splits):
+    """The activation of a single-weight product applies to the whole sum, whoever adds it up."""
+    from mlx_sharding_b200.ops import get_backend
+    C = get_backend("b200").C()
+    gen = torch.Generator("cuda").manual_seed(T)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()
+    x, w, b = r(T, 2048), (r(256, 2048) * 0.03).bfloat16(), r(256)
+    y = x.double() @ w.double().T + b.double()
+    want = y.clamp(min=0).square()
+    mag = x.double().abs() @ w.double().abs().T * 2048 * 2 ** -24
+    got = C.linear(x, w, bias=b, act=4, splits=splits).double()
+    assert ((got - want).abs() <= want * 2 ** -8 + 2 * y.abs() * mag + mag.square() + 1e-6).all()
