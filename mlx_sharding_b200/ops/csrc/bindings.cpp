@@ -147,7 +147,7 @@ int auto_splits(int rows, int n, int k, bool grouped) {
 // ---- GEMM -------------------------------------------------------------------------------------------------------
 Tensor linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& w2, const c10::optional<Tensor>& residual,
               const c10::optional<Tensor>& bias, int64_t act, double softcap, bool out_fp32, const c10::optional<Tensor>& out_,
-              int64_t splits, int64_t signal_flag_ptr, int64_t signal_value, double act_limit, int64_t wait_spins) {
+              int64_t splits, int64_t signal_flag_ptr, int64_t signal_value, double act_limit, int64_t wait_spins, int64_t pair) {
   check_bf16(x, "x"); check_bf16(w, "w"); check_rows(x, "x"); check_rows(w, "w");
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t T = x.size(0), K = x.size(1), N = w.size(0);
@@ -156,7 +156,7 @@ Tensor linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& w2,
   TORCH_CHECK(out.dim() == 2 && out.stride(1) == 1 && out.size(0) >= T && out.size(1) == N, "bad out tensor");
   if (T == 0) return out;
   b200::GemmArgs a;
-  a.wait = wait_bound(wait_spins);
+  a.wait = wait_bound(wait_spins); a.pair = (int)pair;
   a.x = x.data_ptr(); a.x_rows = T; a.ld_x = x.stride(0);
   a.w = w.data_ptr(); a.ld_w = w.stride(0);
   if (w2.has_value()) { check_bf16(*w2, "w2"); TORCH_CHECK(w2->sizes() == w.sizes() && w2->stride(0) == w.stride(0)); a.w2 = w2->data_ptr(); }
@@ -188,7 +188,7 @@ Tensor grouped_linear(const Tensor& x, const Tensor& w, const c10::optional<Tens
                       int64_t max_rows, int64_t act, bool out_fp32, const c10::optional<Tensor>& row_dst,
                       const c10::optional<Tensor>& signal_peers, const c10::optional<Tensor>& done_counter, int64_t expected_rows,
                       int64_t expert_stride, int64_t ep_arrive_ptr, const c10::optional<Tensor>& ep_seq, int64_t ep_error_ptr,
-                      int64_t ep_world, bool ep_zero_other, double act_limit) {
+                      int64_t ep_world, bool ep_zero_other, double act_limit, int64_t pair) {
   check_bf16(x, "x"); check_bf16(w, "w"); check_rows(x, "x");
   TORCH_CHECK(w.dim() == 3 && w.is_contiguous(), "w must be contiguous [E, N, K]");
   const c10::cuda::CUDAGuard guard(x.device());
@@ -204,7 +204,7 @@ Tensor grouped_linear(const Tensor& x, const Tensor& w, const c10::optional<Tens
   Tensor out = torch::empty({ep_ret ? 0 : R, N}, x.options().dtype(out_fp32 ? torch::kFloat32 : torch::kBFloat16));
   if (R == 0) return out;
   b200::GemmArgs a;
-  a.wait = wait_bound();
+  a.wait = wait_bound(); a.pair = (int)pair;
   a.x = x.data_ptr(); a.x_rows = R; a.ld_x = x.stride(0);
   a.w = w.data_ptr(); a.ld_w = K;
   if (w2.has_value()) { check_bf16(*w2, "w2"); TORCH_CHECK(w2->is_contiguous() && w2->sizes() == w.sizes()); a.w2 = w2->data_ptr(); }
@@ -1667,13 +1667,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear", &linear, py::arg("x"), py::arg("w"), py::arg("w2") = py::none(), py::arg("residual") = py::none(),
         py::arg("bias") = py::none(), py::arg("act") = 0, py::arg("softcap") = 0.0, py::arg("out_fp32") = false,
         py::arg("out") = py::none(), py::arg("splits") = 0, py::arg("signal_flag_ptr") = 0, py::arg("signal_value") = 0, py::arg("act_limit") = 0.0,
-        py::arg("wait_spins") = (int64_t)b200::kWaitSpins);
+        py::arg("wait_spins") = (int64_t)b200::kWaitSpins, py::arg("pair") = -1);
   m.def("check_waits", &check_waits);
   m.def("grouped_linear", &grouped_linear, py::arg("x"), py::arg("w"), py::arg("w2") = py::none(), py::arg("expert_offsets"),
         py::arg("max_rows"), py::arg("act") = 0, py::arg("out_fp32") = false, py::arg("row_dst") = py::none(),
         py::arg("signal_peers") = py::none(), py::arg("done_counter") = py::none(), py::arg("expected_rows") = 0,
         py::arg("expert_stride") = 0, py::arg("ep_arrive_ptr") = 0, py::arg("ep_seq") = py::none(), py::arg("ep_error_ptr") = 0,
-        py::arg("ep_world") = 0, py::arg("ep_zero_other") = false, py::arg("act_limit") = 0.0);
+        py::arg("ep_world") = 0, py::arg("ep_zero_other") = false, py::arg("act_limit") = 0.0, py::arg("pair") = -1);
   m.def("linear_q", &linear_q);
   m.def("grouped_linear_q", &grouped_linear_q);
   m.def("gemm_q_supported", &gemm_q_supported);

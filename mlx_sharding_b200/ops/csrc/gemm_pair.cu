@@ -12,8 +12,9 @@
 //     staging in shared memory, no barrier; the residual is added in fp32 before the only rounding.
 // Roles (384 threads per CTA): warp 0 TMA, warp 1 MMA (leader CTA) + TMEM, warps 4..11 epilogue.
 // B200, whole blocks, one-SM tiles -> pairs: Llama-3-8B feed-forward on 8 k tokens (power-capped) 2804 -> 2432 us, its attention on 4 k tokens 533 -> 461 us,
-// DeepSeek-V2-Lite attention on 64 x ~128 tokens 382 -> 333 us, Gemma-2-9B attention on 2 k tokens 273 -> 248 us.  Up to 256 rows the one-SM kernel is
-// as good (it streams the weight once either way), and results that go to peer memory (stage hand-off, expert-parallel return) stay with it.
+// DeepSeek-V2-Lite attention on 64 x ~128 tokens 382 -> 333 us, Gemma-2-9B attention on 2 k tokens 273 -> 248 us.  A launch costs ~4 us more than one of the
+// one-SM kernel, and the gate / up epilogue is exposed (one accumulator set of 512 columns): pair_pays below.  Up to 256 rows the one-SM kernel is as
+// good (it streams the weight once either way), and results that go to peer memory (stage hand-off, expert-parallel return) stay with it.
 #include <algorithm>
 
 #include "gemm_cluster.cuh"
@@ -306,11 +307,41 @@ cudaError_t pair_launch_one(const CUtensorMap& tw, const CUtensorMap& tw2, const
 
 }  // namespace
 
+// Where pairs are faster.  Both kernels walk their tiles in rounds of the chip; times fitted to 378 products whose weights come from HBM (257 to 8192 rows,
+// 22 weights of 256 x 2048 to 14336 x 4096; 6 % rms), us, kb = k-blocks of 64:
+//   one weight:   one SM 2.6 + rounds (2.5 + 0.355 kb), pairs 6.7 + rounds (0.95 + 0.327 kb); the one-SM kernel's partly filled last token tile costs
+//                 in proportion.  3648 x 2048: 1024 rows 17.3 / 19.4, 4096 rows 52 / 48; 6144 x 4096: 512 rows 29.7 / 31.0, 2048 rows 79 / 71; 10944 x 2048: 320 rows
+//                 26.5 / 29.0, 8192 rows 308 / 242.  Below a gain of 3 % the smaller launch stays.
+//   + residual:   pairs always (with one the one-SM kernel takes 6 us more a round): 2048 x 2048, 257 rows 22.4 / 18.3, 8192 rows 113 / 56
+//   gate and up:  one SM rounds (7.8 + 0.72 kb), pairs 1 + rounds (15.7 + 0.59 kb), the exposed epilogue: 10944 x 2048 stays behind up to 8192 rows (51 / 70 at
+//                 257, 157 / 177 at 2048, 632 / 646 at 8192), 14336 x 3584 is ahead from three rounds on (157 / 126 at 513, 359 / 338 at 2048), 14336 x 4096 too
+//                 (146 / 138 at 513, 211 / 212 at 1024, 405 / 372 at 2048; two rounds: 108 / 113)
+// Experts: a pair's products are as wide as the rows a tile holds, the one-SM kernel's always 256, and it looks at every tile that could exist.  gate / up of
+// 66 x 1408 x 2048, top 6 and two for all: 600 rows 201 / 160, 2048 rows 260 / 243; 8 x 2048 x 2048, top 2 (full tiles on average): 1024 rows 62 / 74, 8192 rows 246 / 277,
+// between (tiles two thirds full): 800 rows 58 / 42, 1300 rows 82 / 73; long K either way: 8 x 14336 x 4096, 1024 rows 617 / 571.  Down (fp32 results): 66 x 2048 x 1408, 2048 rows
+// 113 / 105, 8 x 4096 x 14336, 2048 rows 650 / 449, but 32 x 2048 x 1024, 2048 rows 82 / 92, and 8 x 2048 x 2048, 1024 rows 34 / 40.
+static bool pair_pays(const GemmArgs& a) {
+  auto up = [](long long x, long long y) { return (x + y - 1) / y; };
+  const int kb = (int)up(a.k, kBlockK);
+  if (a.expert_offsets != nullptr) {
+    const double rows = static_cast<double>(a.m) / a.num_experts;                                // of an expert, on average
+    const bool loose = rows < 0.75 * kPairTok * up((long long)rows + 1, kPairTok), many = a.num_experts >= 32;
+    return a.w2 != nullptr ? kb >= 56 || many || loose : kb >= 20 && (kb >= 64 || many || loose);
+  }
+  if (a.residual != nullptr) return true;
+  constexpr int kSms = 148;                                                                      // of the measured chip: rounds
+  const long long pairs = up(up(a.n, kPairFeat) * up(a.m, kPairTok), kSms / 2);
+  if (a.w2 != nullptr) return kb >= 56 && pairs >= 3;
+  const long long ones = up(up(a.n, kTileM) * a.m, (long long)kPairTok * kSms);
+  return 6.7 + pairs * (0.95 + 0.327 * kb) < 0.97 * (2.6 + ones * (2.5 + 0.355 * kb));
+}
+
 bool gemm_pair_takes(const GemmArgs& a) {
   const bool grouped = a.expert_offsets != nullptr;
   if (a.signal_flag != nullptr || a.signal_peers != nullptr || a.row_dst != nullptr || a.ep_arrive != nullptr) return false;
   if (grouped ? (a.expert_stride > 0 || a.num_experts > kPairMaxExperts || a.bn != kPairTok) : a.m <= kPairTok) return false;
   if (a.n <= kTileM || (reinterpret_cast<uintptr_t>(a.out) & 3) != 0 || (reinterpret_cast<uintptr_t>(a.residual) & 3) != 0) return false;
+  if (a.pair == 0 || (a.pair < 0 && !pair_pays(a))) return false;
   return (a.k % 8) == 0 && (a.n % 8) == 0 && (a.ld_out % 2) == 0 && (a.residual == nullptr || (a.ld_res % 2) == 0) && !(a.w2 != nullptr && a.out_fp32);
 }
 

@@ -87,6 +87,7 @@ struct GemmArgs {
   bool persistent = true;                 // splits == 1: persistent kernel (gemm_persistent.cu)
   bool cluster_splitk = true;             // prefer the DSMEM reduction when it applies (decode shapes)
   WaitBound wait;                         // of the waits of gemm_pair.cu
+  int pair = -1;                          // many rows: 1 pairs of SMs where they can, 0 single SMs, -1 by the rule of gemm_pair.cu
   int q_bits = 0, q_group = 64;
   const void* q_scales_t = nullptr; const void* q_biases_t = nullptr;
   const void* q_scales2_t = nullptr; const void* q_biases2_t = nullptr;
@@ -96,7 +97,7 @@ int gemm_pick_bn(int max_rows);
 size_t gemm_workspace_floats(const GemmArgs& a, int bn, int splits);
 cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream);
 cudaError_t gemm_persistent_launch(const GemmArgs& a, cudaStream_t stream);
-bool gemm_pair_takes(const GemmArgs& a);                                     // many rows, no peer-memory epilogue (gemm_pair.cu)
+bool gemm_pair_takes(const GemmArgs& a);                                     // many rows, no peer-memory epilogue, and faster (gemm_pair.cu)
 cudaError_t gemm_pair_launch(const GemmArgs& a, cudaStream_t stream);
 bool gemm_q_supported(int bits, int group, int k);
 cudaError_t gemm_q_launch(const GemmArgs& a, cudaStream_t stream);

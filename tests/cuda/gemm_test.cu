@@ -89,6 +89,7 @@ static int run_case(const Case& c) {
   a.m = c.m; a.n = c.n; a.k = c.k; a.max_rows = max_rows; a.num_experts = c.E; a.expert_offsets = d_offs;
   a.out = out; a.ld_out = c.n; a.out_fp32 = c.fp32; a.residual = res; a.ld_res = c.n; a.bias = bias;
   a.act = c.act; a.softcap = c.softcap; a.bn = c.bn; a.splits = c.splits;
+  a.pair = c.name.rfind("pair", 0) == 0 ? 1 : -1;
   int bn = c.bn > 0 ? c.bn : gemm_pick_bn(max_rows);
   float* ws = nullptr; unsigned int* ctr = nullptr;
   if (c.splits > 1) {

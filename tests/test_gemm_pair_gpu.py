@@ -33,24 +33,24 @@ def test_dense(C, T, N, K, kind):
     w, w2 = rnd(N, K, seed=2, scale=K ** -0.5), rnd(N, K, seed=3, scale=K ** -0.5)
     y, mag = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     if kind == "plain":
-        close(C.linear(x, w, None, None, None, 0, 0.0, False, None, 0, 0, 0), y, mag, K)
+        close(C.linear(x, w, None, None, None, 0, 0.0, False, None, 0, 0, 0, pair=1), y, mag, K)
     elif kind == "fp32":
-        got = C.linear(x, w, None, None, None, 0, 0.0, True, None, 0, 0, 0)
+        got = C.linear(x, w, None, None, None, 0, 0.0, True, None, 0, 0, 0, pair=1)
         assert got.dtype == torch.float32 and ((got.double() - y).abs() <= mag * K ** 0.5 * 2 ** -22 + 1e-6).all()
     elif kind == "residual_bias":
         r, b = rnd(T, N + 2, seed=4)[:, :N], rnd(N, seed=5)
         out = torch.zeros(T + 1, N + 6, dtype=torch.bfloat16, device="cuda")[:, 2:N + 2]
-        C.linear(x, w, None, r, b, 0, 0.0, False, out, 0, 0, 0)
+        C.linear(x, w, None, r, b, 0, 0.0, False, out, 0, 0, 0, pair=1)
         close(out[:T], y + r.double() + b.double(), mag, K)
         assert (out[T] == 0).all()
     elif kind == "relu2":
         ref = y.clamp(min=0).square()
-        got = C.linear(x, w, None, None, None, 4, 0.0, False, None, 0, 0, 0).double()
+        got = C.linear(x, w, None, None, None, 4, 0.0, False, None, 0, 0, 0, pair=1).double()
         assert ((got - ref).abs() <= ref * 2 ** -8 + 2 * y.abs() * mag * K ** 0.5 * 2 ** -22 + 1e-5).all()
     else:
         u, mu = x.double() @ w2.double().t(), x.double().abs() @ w2.double().abs().t()
         ref = y * torch.sigmoid(y) * u
-        got = C.linear(x, w, w2, None, None, 1, 0.0, False, None, 0, 0, 0).double()
+        got = C.linear(x, w, w2, None, None, 1, 0.0, False, None, 0, 0, 0, pair=1).double()
         # the products' errors enter through both factors (|d silu| <= 1.1); the hardware's exp and division are good to 2^-20
         assert ((got - ref).abs() <= ref.abs() * (2 ** -8 + 2 ** -18) + (1.1 * u.abs() * mag + y.abs() * mu) * K ** 0.5 * 2 ** -22 + 1e-5).all()
 
@@ -61,8 +61,8 @@ def test_grouped(C, rows, N, K):
     E, T = len(rows), max(rows)
     offs = torch.tensor([0] + rows).cumsum(0).to(torch.int32).cuda()
     x, w, w2 = rnd(sum(rows), K, seed=1), rnd(E, N, K, seed=2, scale=K ** -0.5), rnd(E, N, K, seed=3, scale=K ** -0.5)
-    y = C.grouped_linear(x, w, None, offs, T, 0, True).double()
-    h = C.grouped_linear(x, w, w2, offs, T, 1, False).double()
+    y = C.grouped_linear(x, w, None, offs, T, 0, True, pair=1).double()
+    h = C.grouped_linear(x, w, w2, offs, T, 1, False, pair=1).double()
     at = 0
     for e, n in enumerate(rows):
         xs = x[at:at + n].double()
@@ -72,3 +72,19 @@ def test_grouped(C, rows, N, K):
         ref = g * torch.sigmoid(g) * u
         assert ((h[at:at + n] - ref).abs() <= ref.abs() * (2 ** -8 + 2 ** -18) + (1.1 * u.abs() * mag + g.abs() * mu) * K ** 0.5 * 2 ** -22 + 1e-5).all()
         at += n
+
+
+# both sides of the rule's lines: rows in one and two tiles, one round and several, short and long K
+@pytest.mark.parametrize("T,N,K,dual", [(257, 256, 128, False), (320, 10944, 512, False), (640, 10944, 512, False), (1500, 3648, 2048, False), (300, 4096, 14336, False),
+                                        (513, 14336, 3584, True), (512, 14336, 3584, True), (600, 1408, 2048, True)])
+def test_rule(C, T, N, K, dual):
+    """Pairs of SMs, single SMs, and whichever the rule takes."""
+    x, w, w2 = rnd(T, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(N, K, seed=3, scale=K ** -0.5) if dual else None
+    one, two, auto = (C.linear(x, w, w2, act=1 if dual else 0, pair=p) for p in (0, 1, -1))
+    assert torch.equal(auto, one) or torch.equal(auto, two)
+    y, mag = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    if dual:
+        u, mu = x.double() @ w2.double().t(), x.double().abs() @ w2.double().abs().t()
+        y, mag = y * torch.sigmoid(y) * u, 1.1 * u.abs() * mag + y.abs() * mu
+    for got in (one, two):
+        assert ((got.double() - y).abs() <= y.abs() * (2 ** -8 + 2 ** -18) + mag * K ** 0.5 * 2 ** -22 + 1e-5).all()

@@ -53,7 +53,7 @@ def test_many_row_gemm_returns(C, dual, fp32):
     g = torch.Generator(device="cuda").manual_seed(0)
     rnd = lambda *s: (torch.randn(*s, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
     x, w, w2 = rnd(5000, 1024), rnd(4096, 1024), rnd(4096, 1024) if dual else None
-    call = lambda **kw: C.linear(x, w, w2, act=1 if dual else 0, out_fp32=fp32, **kw)
+    call = lambda **kw: C.linear(x, w, w2, act=1 if dual else 0, out_fp32=fp32, pair=1, **kw)
     want = call()
     torch.cuda.synchronize()
     for spins in (0, 3, 20):
