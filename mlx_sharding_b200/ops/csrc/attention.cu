@@ -346,14 +346,14 @@ cudaError_t launch_vector(const PagedAttnArgs& a, cudaStream_t s) {
 
 // Where the vector form is faster.  B200, us, vector / matrix form, by the bound of the contexts: one query head per kv head, 16 heads of 192 / 128, 1 token
 // 2.2 / 2.7 (up to 16 keys; 17: 3.2 / 2.7), 8 tokens 2.4 / 2.8 (16; 17: 3.3 / 3.2), 64 tokens 3.0 / 3.7 (1), 3.9 / 3.8 (8), 5.1 / 3.8 (16), 256 tokens 8.5 / 11.1 (8), 11.7 / 11.1 (16),
-// 1024 tokens 42.8 / 45.7 (16), 54.2 / 53.6 (17); 32 heads of 128, 1 token 2.3 / 2.5 (16), 8 tokens 2.5 / 2.7 (8), 2.8 / 2.6 (16), 64 tokens 4.9 / 5.0 (8), 256 tokens 14.1 / 12.9 (8);
+// 1024 tokens 42.8 / 45.7 (16), 54.2 / 53.6 (17); 32 heads of 128, 1 token 2.3 / 2.5 (16), 8 tokens 2.5 / 2.7 (8), 2.8 / 2.6 (16), 64 tokens 4.9 / 5.0 (8), 256 tokens 11.7 / 12.9 (1), 14.1 / 12.9 (8);
 // 16 heads of 256, 8 tokens 2.6 / 3.0 (16), 64 tokens 3.8 / 4.5 (8), 5.2 / 4.5 (16), 6.0 / 7.5 (17), 8.0 / 7.5 (32), 1024 tokens 71 / 77 (17), 96 / 90 (32); two query heads
 // per kv head, 8 of 256, 64 tokens 4.3 / 4.5 (8), 5.0 / 4.5 (16), 256 tokens 10.6 / 8.4 (8).  Heads of 64 and larger groups: the matrix form is as fast or faster from one key on.
 bool vector_form(int dk, int G, int max_ctx, long long pairs) {
   if (max_ctx <= 0 || max_ctx > 24) return false;
   if (G == 2 && dk == 256) return max_ctx <= 8 && pairs <= 512;
   if (G != 1 || dk < 128) return false;
-  if (max_ctx <= 8) return dk > 128 || pairs <= 2048;
+  if (max_ctx <= 8) return dk > 128 || pairs <= 2048 || max_ctx <= 2;
   if (max_ctx <= 16) return pairs <= (dk > 128 ? 128 : 32) || (dk == 192 && pairs >= 8192);
   return dk == 256 && pairs >= 1024;
 }
