@@ -16,13 +16,13 @@
 //   * S is double buffered, the scores of each stream and the second products have an issuing thread of their own (issuing, not the tensor pipe, was
 //     what one thread for all was bound by: ~100 cycles per product), so scores run a tile ahead of the softmax warps; P overwrites its own score buffer.  A buffer is written again only after the product that reads
 //     it has completed (its commit is waited for);
-//   * one thread per row: no shuffles; the running maximum may lag by 2^8 before the accumulator in TMEM is rescaled, so rescales are rare after
-//     the first tiles;
-//   * probabilities enter the second product as two bf16 terms (error 2^-17 of each, where a lagging maximum leaves no probability exact; a visible
-//     infinity in V gives NaN, as the low term may be 0 or of the other sign).  One term costs half of the second product's tensor time, but with the lag
-//     its error alone is above the result's rounding: error of the op against 64 bits at scores with a spread of 2: mma.sync form (maximum exact, one
-//     term) 1.838e-3, one term and the lag 2.104e-3, one term and no lag 1.838e-3, two terms and the lag 1.647e-3.  B200, Llama-3-8B heads 2 x 2 k / 1 x
-//     8 k tokens, DeepSeek-V2-Lite 2 k behind 6 k: 101 / 475 / 143 us, 122 / 577 / 176 without the lag, 106 / 565 / 166 with two terms;
+//   * one thread per row: no shuffles; the accumulator in TMEM is rescaled when a row of the warp has a new maximum;
+//   * capped scores, heads of 256 and SINK (fp32 probabilities, or queries, before): probabilities enter the second product as two bf16 terms (error 2^-17 of
+//     each; a visible infinity in V gives NaN, as the low term may be 0 or of the other sign), and the maximum may lag by 2^8 before a rescale.  The plain modes
+//     have one term, and with it the exact maximum, as the mma.sync form: the dominant probability is then 1 and rounds to itself, which the lag would
+//     lose.  Error of the op against 64 bits at scores with a spread of 2: mma.sync form 1.838e-3, one term and the lag 2.104e-3, one term and the exact maximum
+//     1.838e-3, two terms 1.647e-3 (the rounding of the result: 1.645e-3).  B200, whole blocks, lag / exact / two terms: Llama-3-8B 4 k tokens of prompts 433 / 447
+//     / 450 us, DeepSeek-V2-Lite 2 k behind 6 k 301 / 314 / 340 us, 64 x ~128 315 / 312 / 318 us (the low terms cost tensor time and, under the power cap, clock);
 //   * heads of 256 (Gemma-2): the accumulator takes 256 columns, so there is one stream, whose rows' 64 scores are shared by two threads, and
 //     three score buffers;
 //   * MLA: the decompressed keys / values are read where the kv_b product left them ([rows, heads * (nope + v)]), the shared rotary key from
@@ -30,10 +30,10 @@
 //   * SINK (windowed attention of the hybrid stacks, sinkattn.cu): only tiles with visible keys are walked; the fp32 queries enter the first product
 //     as two bf16 terms (the softmax warps lay them out in shared memory), a sink joins the denominator, gates multiply the result.
 // Rows of V behind the last key are zeroed in shared memory (what lies there may be anything, and 0 * inf is not 0).
-// B200, the kernel alone, one CTA per item with one issuing thread -> this form: Llama-3-8B heads, 1 x 8 k tokens 753 -> 496 us (1109 TFLOP/s), 2 x 2 k
-// 145 -> 104 us, 64 x 128 75 -> 53 us; DeepSeek-V2-Lite 2 k behind 6 k 213 -> 150 us; windowed attention with a sink (mma.sync form before), 4 k
-// tokens of 16 heads, window 1024, 241 -> 91 us.  Before that, the mma.sync form: 2 x 2 k tokens 430 us, the portion 867 us; capped scores ran on the
-// decode kernel (2 x 1 k tokens of Gemma-2-9B 1853 us, here 53 us).
+// B200, the kernel alone, one CTA per item with one issuing thread and a lagging maximum -> this form: Llama-3-8B heads, 1 x 8 k tokens 753 -> 577 us
+// (953 TFLOP/s), 2 x 2 k 145 -> 122 us, 64 x 128 75 -> 54 us; DeepSeek-V2-Lite 2 k behind 6 k 213 -> 176 us; windowed
+// attention with a sink (mma.sync form before), 4 k tokens of 16 heads, window 1024, 241 -> 89 us.  Before that, the mma.sync form: 1 x 8 k tokens 2869 us, 2 x 2 k
+// 439 us, the portion 864 us; capped scores ran on the decode kernel (2 x 1 k tokens of Gemma-2-9B 1814 us, here 52 us).
 #include <cuda.h>
 
 #include "gemm_tmap.h"
@@ -50,7 +50,7 @@ constexpr int kRows = 128;                    // query rows of a stream (UMMA M)
 constexpr int kKeys = 64;                     // keys of a tile
 constexpr int kFlashThreads = 384;            // warps 0..7: softmax, 8: TMA + item list, 9 / 10: S of a stream (9: TMEM too), 11: P V
 constexpr int kSlots = 4;                     // items that the producer may be ahead
-constexpr float kLazy = 8.f;                  // how far (log2) the maximum may lag
+constexpr float kLazy = 8.f;                  // how far (log2) the maximum may lag where probabilities are two terms
 
 constexpr int kMaxSeqs = 512;                 // sequences of a step that the item table holds
 
@@ -71,6 +71,8 @@ struct FlashTcParams {
   WaitBound wait;
 };
 
+// probabilities in two terms and a maximum that may lag, or in one and the exact maximum
+__host__ __device__ constexpr bool ft_split(int dv, int mode) { return dv > 128 || (mode & (kCap | kSink)) != 0; }
 __host__ __device__ constexpr int ft_streams(int dv) { return dv > 128 ? 1 : 2; }
 __host__ __device__ constexpr int ft_bufs(int dv) { return dv > 128 ? 3 : 2; }
 __host__ __device__ constexpr int ft_stages(int dk, int dv, int mode) { return (mode & kSink) || dk + dv > 320 ? 2 : dk + dv > 256 ? 3 : 4; }
@@ -171,11 +173,12 @@ template <int DK, int DV, int MODE>
 __global__ void __launch_bounds__(kFlashThreads, 1)
 flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                 const __grid_constant__ CUtensorMap tmap_pe, const FlashTcParams p) {
-  constexpr bool MLA = (MODE & kMla) != 0, CAP = (MODE & kCap) != 0, SINK = (MODE & kSink) != 0;
+  constexpr bool MLA = (MODE & kMla) != 0, CAP = (MODE & kCap) != 0, SINK = (MODE & kSink) != 0, SPLIT = ft_split(DV, MODE);
   constexpr int NS = ft_streams(DV), NB = ft_bufs(DV), ST = ft_stages(DK, DV, MODE);
   constexpr int CK = DK / 64, CV = DV / 64;
   constexpr int QB = ft_q_bytes(DK, MODE), KB = kKeys * DK * 2, VB = kKeys * DV * 2, CHUNK = kKeys * 128;
   constexpr uint32_t O_COL = NS * NB * 64;
+  constexpr float LAG = SPLIT ? kLazy : 0.f;
   static_assert(O_COL + NS * DV <= 512, "TMEM budget exceeded");
   constexpr uint32_t IDESC_S = ft_idesc(kRows, kKeys, 0), IDESC_O = ft_idesc(kRows, DV, 1);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -416,7 +419,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             for (int ks = 0; ks < kKeys / 16; ++ks) {
               const uint64_t bd = umma_desc_mn_sw128(va + ks * 2048, CHUNK, 1024);
               umma_f16_ts(d, pa + 8 * ks, bd, IDESC_O, (j | ks) ? 1u : 0u);
-              umma_f16_ts(d, pa + 32 + 8 * ks, bd, IDESC_O, 1u);
+              if constexpr (SPLIT) umma_f16_ts(d, pa + 32 + 8 * ks, bd, IDESC_O, 1u);
             }
             umma_commit(&o_done[s * NB + g[s] % NB]);
             ++g[s];
@@ -515,8 +518,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           top = fmaxf(top, red[(half ^ 1) * kRows + row]);
         }
         top *= sl2;
-        if (__any_sync(0xffffffffu, top > m + kLazy)) {                          // (m = -inf: the row's first visible tile)
-          const float mn = top > m + kLazy ? top : m;
+        if (__any_sync(0xffffffffu, top > m + LAG)) {                          // (m = -inf: the row's first visible tile)
+          const float mn = top > m + LAG ? top : m;
           const float corr = mn == -INFINITY ? 1.f : exp2f(m - mn);
           m = mn;
           l *= corr;
@@ -537,20 +540,20 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         const float sub = m == -INFINITY ? 0.f : -m;
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t hi[PAIRS], lo[PAIRS];
+        uint32_t hi[PAIRS], lo[SPLIT ? PAIRS : 1];
 #pragma unroll
         for (int c = 0; c < PAIRS; ++c) {
           const float a = exp2f(fmaf(x[2 * c], sl2, sub)), b = exp2f(fmaf(x[2 * c + 1], sl2, sub));
           sum[c & 3] += a + b;
           hi[c] = pack_bf16(a, b);
-          lo[c] = pack_bf16(a - bf16_lo(hi[c]), b - bf16_hi(hi[c]));
+          if constexpr (SPLIT) lo[c] = pack_bf16(a - bf16_lo(hi[c]), b - bf16_hi(hi[c]));
         }
         l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
         if constexpr (NS == 1) named_bar_sync(2, 256);                           // P overwrites the scores: both halves of a row have been read
 #pragma unroll
         for (int c = 0; c < PAIRS; c += 16) {
           tmem_st16(buf + half * PAIRS + c, hi + c);
-          tmem_st16(buf + 32 + half * PAIRS + c, lo + c);
+          if constexpr (SPLIT) tmem_st16(buf + 32 + half * PAIRS + c, lo + c);
         }
         tmem_st_wait();
         const int vend = v_end - tile0;
