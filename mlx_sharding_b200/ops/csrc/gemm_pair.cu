@@ -307,33 +307,44 @@ cudaError_t pair_launch_one(const CUtensorMap& tw, const CUtensorMap& tw2, const
 
 }  // namespace
 
-// Where pairs are faster.  Both kernels walk their tiles in rounds of the chip; times fitted to 378 products whose weights come from HBM (257 to 8192 rows,
-// 22 weights of 256 x 2048 to 14336 x 4096; 6 % rms), us, kb = k-blocks of 64:
-//   one weight:   one SM 2.6 + rounds (2.5 + 0.355 kb), pairs 6.7 + rounds (0.95 + 0.327 kb); the one-SM kernel's partly filled last token tile costs
-//                 in proportion.  3648 x 2048: 1024 rows 17.3 / 19.4, 4096 rows 52 / 48; 6144 x 4096: 512 rows 29.7 / 31.0, 2048 rows 79 / 71; 10944 x 2048: 320 rows
-//                 26.5 / 29.0, 8192 rows 308 / 242.  Below a gain of 3 % the smaller launch stays.
-//   + residual:   pairs always (with one the one-SM kernel takes 6 us more a round): 2048 x 2048, 257 rows 22.4 / 18.3, 8192 rows 113 / 56
-//   gate and up:  one SM rounds (7.8 + 0.72 kb), pairs 1 + rounds (15.7 + 0.59 kb), the exposed epilogue: 10944 x 2048 stays behind up to 8192 rows (51 / 70 at
-//                 257, 157 / 177 at 2048, 632 / 646 at 8192), 14336 x 3584 is ahead from three rounds on (157 / 126 at 513, 359 / 338 at 2048), 14336 x 4096 too
-//                 (146 / 138 at 513, 211 / 212 at 1024, 405 / 372 at 2048; two rounds: 108 / 113)
-// Experts: a pair's products are as wide as the rows a tile holds, the one-SM kernel's always 256, and it looks at every tile that could exist.  gate / up of
-// 66 x 1408 x 2048, top 6 and two for all: 600 rows 201 / 160, 2048 rows 260 / 243; 8 x 2048 x 2048, top 2 (full tiles on average): 1024 rows 62 / 74, 8192 rows 246 / 277,
-// between (tiles two thirds full): 800 rows 58 / 42, 1300 rows 82 / 73; long K either way: 8 x 14336 x 4096, 1024 rows 617 / 571.  Down (fp32 results): 66 x 2048 x 1408, 2048 rows
-// 113 / 105, 8 x 4096 x 14336, 2048 rows 650 / 449, but 32 x 2048 x 1024, 2048 rows 82 / 92, and 8 x 2048 x 2048, 1024 rows 34 / 40.
+// Where pairs are faster.  Both kernels walk their tiles in rounds of the chip; times from products with both kernels in turn in one process, weights from HBM,
+// 257 to 8192 rows, us, single SMs / pairs, kb = k-blocks of 64:
+//   bf16:        single SMs 2.6 + rounds (2.5 + 0.355 kb), pairs 6.7 + rounds (0.95 + 0.327 kb), at least 6.5 a round (the epilogue); the single SMs' partly filled
+//                last token tile costs in proportion.  3648 x 2048: 1024 rows 17.3 / 19.2, 4096 rows 53 / 49; 4096 x 512: 8192 rows 43 / 52; 6144 x 4096: 512 rows 31 / 33,
+//                2048 rows 81 / 72; 10944 x 2048: 384 rows 27 / 29, 8192 rows 312 / 245.  Below a gain of 3 % the smaller launch stays.
+//   + residual:  pairs (with one, single SMs take 6 us more a round): 256 x 2048 21 / 18, 2048 x 2048 at 257 rows 23 / 19, 8192 rows 112 / 56
+//   fp32:        pairs' last epilogue is exposed: single SMs 1 + rounds (2.5 + 0.38 kb), pairs 14 + rounds (3 + 0.31 kb).  4096 x 2048: 1024 rows 21 / 29, 8192 rows
+//                118 / 115; 2048 x 4096: 2048 rows 28 / 35, 8192 rows 115 / 105
+//   gate and up: 256 x 256 of both weights fill TMEM, so every epilogue is exposed (8 us a round more); worth it only where single SMs read weights that L2
+//                (126 MB) does not keep again for every token tile.  10944 x 2048 (90 MB): 257 rows 51 / 70, 2048 rows 157 / 177, 8192 rows 632 / 646; 4096 x 4096: 1024 rows
+//                56 / 63, 8192 rows 386 / 407; 14336 x 4096 (235 MB): 512 rows 108 / 114, 513 rows 147 / 138, 1024 rows 216 / 213, 2048 rows 412 / 378, 4096 rows 799 / 738
+// Experts (E of them, r rows each on average): a pair's products are as wide as the rows that a tile holds and its list holds the tiles that exist; single SMs' are 256
+// wide and their list holds every tile that could exist, so theirs is the less even one where tiles are few or many.
+//   gate and up: kb >= 56 pairs (8 x 14336 x 4096: r 128 435 / 366, r 1024 1843 / 1728; 16 x 4096 x 4096: r 200 375 / 249), kb < 24 not (32 x 2048 x 1024: r 200 82 / 108).
+//                Between, with kb = 32: E 8 r 150 79 / 39, r 325 85 / 74, r 400 64 / 78, r 512 89 / 106, r 2048 244 / 276; E 32 r 128 61 / 68, r 512 175 / 173; E 64 r 96
+//                171 / 161, r 384 386 / 344, r 562 519 / 554 (1408 x 2048), two of 66 with all rows: r 248 260 / 246, r 496 468 / 423, r 727 655 / 699
+//   down (fp32): kb >= 48 pairs (8 x 4096 x 14336: r 256 374 / 275), kb < 20 not (32 x 2048 x 1024: r 200 45 / 60; 64 x 2048 x 768: r 256 96 / 129).  Between: E 8 x 2048 x 2048
+//                r 150 42 / 26, r 400 36 / 41, r 750 73 / 55; E 32 x 1024 x 2048 r 200 39 / 46, r 375 73 / 66; E 64 x 2048 x 1408 r 96 96 / 76, r 768 369 / 330
 static bool pair_pays(const GemmArgs& a) {
   auto up = [](long long x, long long y) { return (x + y - 1) / y; };
-  const int kb = (int)up(a.k, kBlockK);
+  const int kb = static_cast<int>(up(a.k, kBlockK));
   if (a.expert_offsets != nullptr) {
-    const double rows = static_cast<double>(a.m) / a.num_experts;                                // of an expert, on average
-    const bool loose = rows < 0.75 * kPairTok * up((long long)rows + 1, kPairTok), many = a.num_experts >= 32;
-    return a.w2 != nullptr ? kb >= 56 || many || loose : kb >= 20 && (kb >= 64 || many || loose);
+    const double r = static_cast<double>(a.m) / a.num_experts;
+    const int few = 16, many = 48;
+    if (a.w2 != nullptr) {
+      if (kb >= 56 || kb < 24) return kb >= 56;
+      return a.num_experts <= few ? r <= 340 : a.num_experts >= many && r <= 512;
+    }
+    if (kb >= 48 || kb < 20) return kb >= 48;
+    return a.num_experts >= many || (a.num_experts <= few ? r <= 340 || r >= 700 : r >= 350);
   }
+  if (a.w2 != nullptr) return 4ll * a.n * a.k > (126ll << 20) && a.m > 512;
   if (a.residual != nullptr) return true;
   constexpr int kSms = 148;                                                                      // of the measured chip: rounds
-  const long long pairs = up(up(a.n, kPairFeat) * up(a.m, kPairTok), kSms / 2);
-  if (a.w2 != nullptr) return kb >= 56 && pairs >= 3;
-  const long long ones = up(up(a.n, kTileM) * a.m, (long long)kPairTok * kSms);
-  return 6.7 + pairs * (0.95 + 0.327 * kb) < 0.97 * (2.6 + ones * (2.5 + 0.355 * kb));
+  const double pairs = static_cast<double>(up(up(a.n, kPairFeat) * up(a.m, kPairTok), kSms / 2));
+  const double ones = static_cast<double>(up(up(a.n, kTileM) * a.m, static_cast<long long>(kPairTok) * kSms));
+  if (a.out_fp32) return 14 + pairs * (3 + 0.31 * kb) < 0.97 * (1 + ones * (2.5 + 0.38 * kb));
+  return 6.7 + pairs * std::max(6.5, 0.95 + 0.327 * kb) < 0.97 * (2.6 + ones * (2.5 + 0.355 * kb));
 }
 
 bool gemm_pair_takes(const GemmArgs& a) {
