@@ -1,4 +1,4 @@
-// Causal flash-attention for prefill chunks against the paged KV cache (SURVEY §2.6 K7 "flash_prefill").
+// Causal flash-attention for prefill chunks against the paged KV cache.
 //
 // The reference materialises a dense additive [T, T] mask and calls mx.fast.scaled_dot_product_attention
 // on a contiguous cache (shard/server/model/llama.py:48-59, deepseek_v2.py:47-57).  Here causality is

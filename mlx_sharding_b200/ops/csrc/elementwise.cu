@@ -1,4 +1,4 @@
-// Memory-bound helper kernels of a decoder layer (SURVEY §2.6 K1, K2, K6, K7-append): embedding gather
+// Memory-bound helper kernels of a decoder layer: embedding gather
 // with in-kernel MLX-affine dequant, RMSNorm (+Gemma variant, + post-norm residual), rotary embedding
 // (half-split and interleaved/YaRN), paged KV-cache append (plain and MLA-assembling).
 // The reference gets all of these from MLX Metal kernels (mx.fast.rms_norm / mx.fast.rope / Embedding /

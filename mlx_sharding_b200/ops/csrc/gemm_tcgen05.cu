@@ -1,7 +1,6 @@
 // Swap-AB tcgen05 GEMM for LLM inference on sm_100a:  Y[tokens, N] = X[tokens, K] · W[N, K]^T
 //
-// Implements SURVEY §2.6 K3/K4/K5/K8/K9/K11/K12 (all projection GEMMs, the SwiGLU/GeGLU pair, the MoE
-// grouped GEMMs and the LM head) — ops the reference delegates to MLX Metal matmul / gather_qmm
+// All projection GEMMs, the SwiGLU/GeGLU pair, the MoE grouped GEMMs and the LM head: ops the reference delegates to MLX Metal matmul / gather_qmm
 // (shard/server/model/*.py via mlx_lm blocks).
 //
 // Design (B200-first, not a translation of anything):

@@ -1,4 +1,4 @@
-// Absorbed-latent MLA decode attention on tcgen05 / TMEM (SURVEY §2.6 K7, K5 "weight absorption").
+// Absorbed-latent MLA decode attention on tcgen05 / TMEM.
 //
 // DeepSeek-V2's MLA caches one 512-dim latent c_t (+ a 64-dim roped key) per token.  The reference decompresses it to 16 heads of
 // K 192 / V 128 and caches *that* (shard/server/model/deepseek_v2.py:120-125 -> 5120 values per token per layer).  With W_UK folded

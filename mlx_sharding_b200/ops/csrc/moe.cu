@@ -1,4 +1,4 @@
-// DeepSeek-V2 MoE support kernels (SURVEY §2.6 K10/K11): router (fp32 softmax + greedy / group-limited
+// DeepSeek-V2 MoE support kernels: router (fp32 softmax + greedy / group-limited
 // top-k), token permutation for the grouped GEMM, and the weighted combine fused with the residual and
 // — on the last layer of a stage — with the P2P hand-off flag.  The reference gets this from
 // mlx_lm's MoEGate + SwitchGLU (`mx.gather_qmm`, `(y * scores[..., None]).sum(-2)`); nothing is ported.

@@ -2,7 +2,7 @@
 // mbarrier, TMA (cp.async.bulk.tensor), tcgen05 (alloc / mma / commit / ld / fences), and the
 // system-scope release/acquire primitives of the fused P2P stage boundary.
 //
-// Nothing here comes from the reference (it has no native code, SURVEY §2.3); bit layouts follow the
+// Nothing here comes from the reference (it has no native code); bit layouts follow the
 // PTX ISA as mirrored in cute/arch/mma_sm100_desc.hpp (descriptor unions) of the vendored CUTLASS tree.
 #pragma once
 #include <cuda.h>
