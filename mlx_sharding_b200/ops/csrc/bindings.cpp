@@ -510,10 +510,18 @@ b200::FlashPrefillArgs flash_args(const Tensor& q, const Tensor& kpool, const Te
   a.o_ld_t = (long long)a.q_heads * a.dv_;
   return a;
 }
-// A few short prompts: the mma.sync form, whose 64-row CTAs start without TMEM, tensor maps or an item list.  B200, Llama-3-8B heads, mma.sync / tcgen05:
-// one prompt of 64 tokens 5.9 / 8.1 us, 128 9.4 / 9.7, 256 17.9 / 11.6; 16 prompts of 16 14.5 / 15.8; but 64 of 127 150 / 53.
-bool flash_short(int64_t max_ctx, int64_t tokens, int64_t seqs, int64_t heads) {
-  return max_ctx > 0 && max_ctx < 128 && (tokens / 64 + seqs) * heads <= 6 * sm_count();
+// A few short prompts: the mma.sync form, whose 64-row CTAs start without TMEM, tensor maps or an item list (3 to 4 us against 7 to 9), up to so many heads of
+// sequences (P) as its serial walk of tiles allows, by the longest context.  B200, mma.sync / tcgen05, us: heads of 64, 32 tokens P 512 9.1 / 11.3, 64 tokens P 256
+// 6.6 / 7.0, P 512 10.9 / 9.4, 128 tokens P 128 8.4 / 8.6, P 256 11.2 / 8.8, 256 tokens P 32 10.3 / 10.9, P 64 12.1 / 10.9, 512 tokens P 16 14.7 / 15.2, P 32 19.7 / 15.6; heads of
+// 128, 32 tokens P 384 10.2 / 13.9, P 512 14.9 / 14.1, 64 tokens P 64 7.5 / 7.6, P 128 9.3 / 7.8, 128 tokens P 32 9.3 / 9.4, P 64 12.3 / 9.4 (eight prompts of 127 of Llama-3-8B 19.9 /
+// 10.3), 192 tokens P 16 9.8 / 10.2, P 32 14.0 / 10.3, 256 tokens P 8 11.1 / 11.8, P 16 13.9 / 12.1; 192 / 128, 32 tokens P 256 10.0 / 11.3, 64 tokens P 32 6.4 / 6.8, P 64 8.3 / 6.8,
+// 128 tokens P 16 7.4 / 8.0, P 32 9.7 / 8.1, 192 tokens P 16 11.2 / 10.1.  Its CTAs look for their sequence one by one: 64 sequences of 16 tokens, P 512 14.2 / 11.9.
+bool flash_short(int64_t max_ctx, int64_t seqs, int64_t heads, int dk) {
+  if (max_ctx <= 0 || seqs > (dk <= 64 && max_ctx <= 32 ? 32 : 16)) return false;
+  const int64_t P = seqs * heads;
+  if (dk <= 64) return P <= (max_ctx <= 32 ? 512 : max_ctx <= 64 ? 256 : max_ctx <= 128 ? 128 : max_ctx <= 256 ? 32 : max_ctx <= 512 ? 16 : 0);
+  if (dk <= 128) return P <= (max_ctx <= 32 ? 400 : max_ctx <= 64 ? 64 : max_ctx <= 128 ? 32 : max_ctx <= 192 ? 16 : max_ctx <= 256 ? 8 : 0);
+  return P <= (max_ctx <= 32 ? 256 : max_ctx <= 64 ? 32 : max_ctx <= 128 ? 16 : 0);
 }
 // whether flash_prefill takes these tensors (else: paged_attention).  Capped scores of a handful of keys: the decode kernel (Gemma-2-9B heads, one prompt
 // of 16 tokens 3.8 us there, 11.9 here; 64 tokens 12.2 / 8.2; 16 prompts of 16 20.0 / 20.1).  Both forms keep the maximum of the raw scores, so a score
@@ -543,7 +551,7 @@ Tensor flash_prefill(const Tensor& q, const Tensor& kpool_, const Tensor& vpool_
   a.num_seqs = (int)context_lens.numel(); a.max_tiles = (int)((num_tokens + 63) / 64 + a.num_seqs);
   a.scale = (float)scale; a.out = out.data_ptr(); a.wait = wait_bound(wait_spins);
   const bool mma_sync = softcap == 0.0 && b200::flash_prefill_supported(a.dk_, a.dv_);
-  if (b200::flash_tc_supported(a) && !(mma_sync && flash_short(max_ctx, num_tokens, a.num_seqs, a.q_heads))) {
+  if (b200::flash_tc_supported(a) && !(mma_sync && flash_short(max_ctx, a.num_seqs, a.q_heads, a.dk_))) {
     LAUNCH_OK(b200::flash_tc_launch(a, cur_stream()));
   } else {
     TORCH_CHECK(softcap == 0.0, "flash_prefill: capped scores need pages of 16, 32 or a multiple of 64 tokens, 16-byte aligned rows and at most 512 sequences");

@@ -193,8 +193,8 @@ def test_flash_prefill_many_items(B, H, Hk, dk, dv, cap):
 
 
 # the rules that keep a few short prompts off the tcgen05 kernel, on both sides of each line; heads of 256: decode kernel with one tile per warp and with a ring
-@pytest.mark.parametrize("H,Hk,dk,dv,cap", [(32, 8, 128, 128, 0.0), (16, 16, 192, 128, 0.0), (16, 8, 256, 256, 50.0)])
-@pytest.mark.parametrize("q_lens", [[1, 16], [16] * 16, [32] * 4, [31, 33], [127], [128], [127] * 40])
+@pytest.mark.parametrize("H,Hk,dk,dv,cap", [(32, 8, 128, 128, 0.0), (16, 16, 192, 128, 0.0), (16, 8, 256, 256, 50.0), (8, 2, 64, 64, 0.0)])
+@pytest.mark.parametrize("q_lens", [[1, 16], [16] * 16, [32] * 4, [31, 33], [127], [128], [127] * 40, [129, 3], [65], [60] * 5, [500], [513], [32] * 17])
 def test_short_prompts(B, H, Hk, dk, dv, cap, q_lens):
     ctx0 = [0] * len(q_lens)
     meta, tables, kpool, vpool, rnd = paged(q_lens, ctx0, Hk, dk, dv, 64)
