@@ -144,6 +144,22 @@ int auto_splits(int rows, int n, int k, bool grouped) {
   return s;
 }
 
+// workspace and tickets of a split product, flag and counter of a fused stage boundary (products that need neither look nothing up)
+void gemm_scratch(b200::GemmArgs& a, int rows, int splits, int64_t signal_flag_ptr, int64_t signal_value, const torch::Device& dev) {
+  if (splits <= 1 && signal_flag_ptr == 0) return;
+  Scratch& sc = scratch();
+  unsigned int* ctr = reinterpret_cast<unsigned int*>(sc.get_counters(dev).data_ptr<int>());
+  if (splits > 1) {
+    a.workspace = sc.get_ws((int64_t)b200::gemm_workspace_floats(a, b200::gemm_pick_bn(rows), splits), dev).data_ptr<float>();
+    a.tile_counters = ctr;
+  }
+  if (signal_flag_ptr != 0) {
+    a.signal_flag = reinterpret_cast<uint32_t*>(signal_flag_ptr);
+    a.signal_value = (uint32_t)signal_value;
+    a.done_counter = ctr + 65535;
+  }
+}
+
 // ---- GEMM -------------------------------------------------------------------------------------------------------
 Tensor linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& w2, const c10::optional<Tensor>& residual,
               const c10::optional<Tensor>& bias, int64_t act, double softcap, bool out_fp32, const c10::optional<Tensor>& out_,
@@ -167,19 +183,7 @@ Tensor linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& w2,
   a.act = (int)act; a.act_limit = (float)act_limit; a.softcap = (float)softcap;
   int sp = splits > 0 ? (int)splits : auto_splits((int)T, (int)N, (int)K, false);
   a.splits = sp;
-  auto& sc = scratch();
-  Tensor ctr = sc.get_counters(x.device());
-  if (sp > 1) {
-    const int bn = b200::gemm_pick_bn((int)T);
-    Tensor ws = sc.get_ws((int64_t)b200::gemm_workspace_floats(a, bn, sp), x.device());
-    a.workspace = ws.data_ptr<float>();
-    a.tile_counters = reinterpret_cast<unsigned int*>(ctr.data_ptr<int>());
-  }
-  if (signal_flag_ptr != 0) {
-    a.signal_flag = reinterpret_cast<uint32_t*>(signal_flag_ptr);
-    a.signal_value = (uint32_t)signal_value;
-    a.done_counter = reinterpret_cast<unsigned int*>(ctr.data_ptr<int>()) + 65535;
-  }
+  gemm_scratch(a, (int)T, sp, signal_flag_ptr, signal_value, x.device());
   LAUNCH_OK(b200::gemm_launch(a, cur_stream()));
   return out;
 }
@@ -270,19 +274,7 @@ Tensor linear_q(const Tensor& x, const Tensor& wq, const Tensor& scales_t, const
   static const bool q_splitk = [] { const char* e = std::getenv("MLXB200_Q_SPLITK"); return !(e && e[0] == '0'); }();
   int sp = splits > 0 ? (int)splits : ((q_splitk && T <= 32) ? auto_splits((int)T, (int)N, (int)K, false) : 1);
   a.splits = sp;
-  auto& sc = scratch();
-  Tensor ctr = sc.get_counters(x.device());
-  if (sp > 1) {
-    const int bn = b200::gemm_pick_bn((int)T);
-    Tensor ws = sc.get_ws((int64_t)b200::gemm_workspace_floats(a, bn, sp), x.device());
-    a.workspace = ws.data_ptr<float>();
-    a.tile_counters = reinterpret_cast<unsigned int*>(ctr.data_ptr<int>());
-  }
-  if (signal_flag_ptr != 0) {
-    a.signal_flag = reinterpret_cast<uint32_t*>(signal_flag_ptr);
-    a.signal_value = (uint32_t)signal_value;
-    a.done_counter = reinterpret_cast<unsigned int*>(ctr.data_ptr<int>()) + 65535;
-  }
+  gemm_scratch(a, (int)T, sp, signal_flag_ptr, signal_value, x.device());
   LAUNCH_OK(b200::gemm_q_launch(a, cur_stream()));
   return out;
 }
@@ -513,14 +505,14 @@ b200::FlashPrefillArgs flash_args(const Tensor& q, const Tensor& kpool, const Te
 // A few short prompts: the mma.sync form, whose 64-row CTAs start without TMEM, tensor maps or an item list (3 to 4 us against 7 to 9), up to so many heads of
 // sequences (P) as its serial walk of tiles allows, by the longest context.  B200, mma.sync / tcgen05, us: heads of 64, 32 tokens P 512 9.1 / 11.3, 64 tokens P 256
 // 6.6 / 7.0, P 512 10.9 / 9.4, 128 tokens P 128 8.4 / 8.6, P 256 11.2 / 8.8, 256 tokens P 32 10.3 / 10.9, P 64 12.1 / 10.9, 512 tokens P 16 14.7 / 15.2, P 32 19.7 / 15.6; heads of
-// 128, 32 tokens P 384 10.2 / 13.9, P 512 14.9 / 14.1, 64 tokens P 64 7.5 / 7.6, P 128 9.3 / 7.8, 128 tokens P 32 9.3 / 9.4, P 64 12.3 / 9.4 (eight prompts of 127 of Llama-3-8B 19.9 /
+// 128, 16 tokens P 512 13.8 / 15.0, 32 tokens P 384 10.2 / 13.9, P 512 14.9 / 14.1, 64 tokens P 64 7.5 / 7.6, P 128 9.3 / 7.8, 128 tokens P 32 9.3 / 9.4, P 64 12.3 / 9.4 (eight prompts of 127 of Llama-3-8B 19.9 /
 // 10.3), 192 tokens P 16 9.8 / 10.2, P 32 14.0 / 10.3, 256 tokens P 8 11.1 / 11.8, P 16 13.9 / 12.1; 192 / 128, 32 tokens P 256 10.0 / 11.3, 64 tokens P 32 6.4 / 6.8, P 64 8.3 / 6.8,
 // 128 tokens P 16 7.4 / 8.0, P 32 9.7 / 8.1, 192 tokens P 16 11.2 / 10.1.  Its CTAs look for their sequence one by one: 64 sequences of 16 tokens, P 512 14.2 / 11.9.
 bool flash_short(int64_t max_ctx, int64_t seqs, int64_t heads, int dk) {
   if (max_ctx <= 0 || seqs > (dk <= 64 && max_ctx <= 32 ? 32 : 16)) return false;
   const int64_t P = seqs * heads;
   if (dk <= 64) return P <= (max_ctx <= 32 ? 512 : max_ctx <= 64 ? 256 : max_ctx <= 128 ? 128 : max_ctx <= 256 ? 32 : max_ctx <= 512 ? 16 : 0);
-  if (dk <= 128) return P <= (max_ctx <= 32 ? 400 : max_ctx <= 64 ? 64 : max_ctx <= 128 ? 32 : max_ctx <= 192 ? 16 : max_ctx <= 256 ? 8 : 0);
+  if (dk <= 128) return P <= (max_ctx <= 16 ? 512 : max_ctx <= 32 ? 400 : max_ctx <= 64 ? 64 : max_ctx <= 128 ? 32 : max_ctx <= 192 ? 16 : max_ctx <= 256 ? 8 : 0);
   return P <= (max_ctx <= 32 ? 256 : max_ctx <= 64 ? 32 : max_ctx <= 128 ? 16 : 0);
 }
 // whether flash_prefill takes these tensors (else: paged_attention).  Capped scores of a handful of keys: the decode kernel (Gemma-2-9B heads, one prompt
