@@ -65,7 +65,7 @@ def _worker(rank, world, port, C, half, q):
     if rank == 0:
         for g in range(G):
             hist[g].append(loop.groups[g].tokens.clone())
-        q.put((prompts, [torch.stack(h) for h in hist]))
+        q.put((prompts.numpy(), [torch.stack(h).numpy() for h in hist]))      # (arrays travel whole; a tensor would be fetched from this process, which may have exited)
     dist.barrier()
     dist.destroy_process_group()
 
@@ -80,6 +80,7 @@ def test_decode_loop_send_recv_matches_single_process(C, world, half):
     for p in procs:
         p.start()
     prompts, hist = q.get(timeout=200)
+    prompts, hist = torch.from_numpy(prompts), [torch.from_numpy(h) for h in hist]
     for p in procs:
         p.join(timeout=60)
         assert p.exitcode == 0
