@@ -16,13 +16,14 @@
 //   * S is double buffered, the scores of each stream and the second products have an issuing thread of their own (issuing, not the tensor pipe, was
 //     what one thread for all was bound by: ~100 cycles per product), so scores run a tile ahead of the softmax warps; P overwrites its own score buffer.  A buffer is written again only after the product that reads
 //     it has completed (its commit is waited for);
-//   * one thread per row: no shuffles; the accumulator in TMEM is rescaled when a row of the warp has a new maximum;
+//   * one thread per row: no shuffles; the accumulator in TMEM is rescaled when a row of the warp has a new maximum, after the tile's
+//     exponentials, so that the last product has had their time to complete (rescaled before them: 1 x 8 k tokens 579 us, here 549);
 //   * capped scores, heads of 256 and SINK (fp32 probabilities, or queries, before): probabilities enter the second product as two bf16 terms (error 2^-17 of
 //     each; a visible infinity in V gives NaN, as the low term may be 0 or of the other sign), and the maximum may lag by 2^8 before a rescale.  The plain modes
 //     have one term, and with it the exact maximum, as the mma.sync form: the dominant probability is then 1 and rounds to itself, which the lag would
 //     lose.  Error of the op against 64 bits at scores with a spread of 2: mma.sync form 1.838e-3, one term and the lag 2.104e-3, one term and the exact maximum
-//     1.838e-3, two terms 1.647e-3 (the rounding of the result: 1.645e-3).  B200, whole blocks, lag / exact / two terms: Llama-3-8B 4 k tokens of prompts 433 / 447
-//     / 450 us, DeepSeek-V2-Lite 2 k behind 6 k 301 / 314 / 340 us, 64 x ~128 315 / 312 / 318 us (the low terms cost tensor time and, under the power cap, clock);
+//     1.838e-3, two terms 1.647e-3 (the rounding of the result: 1.645e-3).  B200, whole blocks, lag / exact / two terms: Llama-3-8B 4 k tokens of prompts 428 / 442
+//     / 450 us, DeepSeek-V2-Lite 2 k behind 6 k 297 / 299 / 340 us, 64 x ~128 312 / 307 / 318 us (the low terms cost tensor time and, under the power cap, clock);
 //   * heads of 256 (Gemma-2): the accumulator takes 256 columns, so there is one stream, whose rows' 64 scores are shared by two threads, and
 //     three score buffers;
 //   * MLA: the decompressed keys / values are read where the kv_b product left them ([rows, heads * (nope + v)]), the shared rotary key from
@@ -30,8 +31,8 @@
 //   * SINK (windowed attention of the hybrid stacks, sinkattn.cu): only tiles with visible keys are walked; the fp32 queries enter the first product
 //     as two bf16 terms (the softmax warps lay them out in shared memory), a sink joins the denominator, gates multiply the result.
 // Rows of V behind the last key are zeroed in shared memory (what lies there may be anything, and 0 * inf is not 0).
-// B200, the kernel alone, one CTA per item with one issuing thread and a lagging maximum -> this form: Llama-3-8B heads, 1 x 8 k tokens 753 -> 577 us
-// (953 TFLOP/s), 2 x 2 k 145 -> 122 us, 64 x 128 75 -> 54 us; DeepSeek-V2-Lite 2 k behind 6 k 213 -> 176 us; windowed
+// B200, the kernel alone, one CTA per item with one issuing thread and a lagging maximum -> this form: Llama-3-8B heads, 1 x 8 k tokens 753 -> 549 us
+// (1002 TFLOP/s), 2 x 2 k 145 -> 122 us, 64 x 128 75 -> 54 us; DeepSeek-V2-Lite 2 k behind 6 k 213 -> 166 us; windowed
 // attention with a sink (mma.sync form before), 4 k tokens of 16 heads, window 1024, 241 -> 89 us.  Before that, the mma.sync form: 1 x 8 k tokens 2869 us, 2 x 2 k
 // 439 us, the portion 864 us; capped scores ran on the decode kernel (2 x 1 k tokens of Gemma-2-9B 1814 us, here 52 us).
 #include <cuda.h>
@@ -518,25 +519,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           top = fmaxf(top, red[(half ^ 1) * kRows + row]);
         }
         top *= sl2;
-        if (__any_sync(0xffffffffu, top > m + LAG)) {                          // (m = -inf: the row's first visible tile)
+        const bool moved = __any_sync(0xffffffffu, top > m + LAG);               // (m = -inf: the row's first visible tile)
+        float corr = 1.f;
+        if (moved) {
           const float mn = top > m + LAG ? top : m;
-          const float corr = mn == -INFINITY ? 1.f : exp2f(m - mn);
+          corr = mn == -INFINITY ? 1.f : exp2f(m - mn);
           m = mn;
           l *= corr;
-          if (j > 0) {
-            wait(&o_done[s * NB + (g - 1) % NB], ((g - 1) / NB) & 1);
-            tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < OCOLS; c += 32) {
-              uint32_t o[32];
-              tmem_ld32(o_addr + c, o);
-              tmem_ld_wait();
-#pragma unroll
-              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
-              tmem_st16(o_addr + c, o);
-              tmem_st16(o_addr + c + 16, o + 16);
-            }
-          }
         }
         const float sub = m == -INFINITY ? 0.f : -m;
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
@@ -554,6 +543,23 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (int c = 0; c < PAIRS; c += 16) {
           tmem_st16(buf + half * PAIRS + c, hi + c);
           if constexpr (SPLIT) tmem_st16(buf + 32 + half * PAIRS + c, lo + c);
+        }
+        if (moved && j > 0) {
+          // the accumulator follows the maximum; here the last tile's product has had the time of the exponentials to complete
+          wait(&o_done[s * NB + (g - 1) % NB], ((g - 1) / NB) & 1);
+          tc_fence_after();
+          constexpr int W = OCOLS % 64 == 0 ? 64 : 32;
+#pragma unroll 1
+          for (int c = 0; c < OCOLS; c += W) {
+            uint32_t o[W];
+#pragma unroll
+            for (int e = 0; e < W; e += 32) tmem_ld32(o_addr + c + e, o + e);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < W; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+#pragma unroll
+            for (int e = 0; e < W; e += 16) tmem_st16(o_addr + c + e, o + e);
+          }
         }
         tmem_st_wait();
         const int vend = v_end - tile0;

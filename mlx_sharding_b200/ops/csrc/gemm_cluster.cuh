@@ -81,6 +81,7 @@ __device__ __forceinline__ void cluster_epilogue_reduce_store(const GemmParams& 
   // TB tokens' partials (and residuals) are in flight together: one token at a time, a DSMEM round trip and one to global memory per token were the tail of the
   // kernel.  B200, 64 tokens, 4 splits: 4096 x 4096 14.3 -> 11.4 us, 4096 x 14336 25.7 -> 23.0 us, 2048 x 8192 15.4 -> 12.4 us.
   constexpr int TB = DUAL ? 4 : 8;
+  const bool relu2 = !DUAL && p.act == kActRelu2;
   for (int tb = t0; tb < t1; tb += TB) {
     float gv[TB][8], uv[TB][8], res[TB];
 #pragma unroll
@@ -110,7 +111,7 @@ __device__ __forceinline__ void cluster_epilogue_reduce_store(const GemmParams& 
       }
       float y = g + bias;
       if (DUAL) y = gated_act(p.act, p.act_limit, y, u);
-      else if (p.act == kActRelu2) { y = fmaxf(y, 0.f); y *= y; }
+      else if (relu2) { y = fmaxf(y, 0.f); y *= y; }
       if (p.softcap > 0.f) y = p.softcap * tanhf(y / p.softcap);
       if (f_glob >= p.n) continue;
       const size_t row = static_cast<size_t>(row_base + t);
