@@ -87,7 +87,7 @@ struct Scratch {
   Tensor counters;           // uint32 tile tickets (self-resetting) + done counters
   Tensor get_ws(int64_t floats, const torch::Device& dev) {
     if (!ws.defined() || ws.numel() < floats) {
-      int64_t n = std::max<int64_t>(floats, 4 << 20);
+      const int64_t n = std::max<int64_t>(floats, captured ? 16 << 20 : 1 << 18);   // (eager: out of the segments that the stream has anyway)
       ws = torch::empty({n}, torch::dtype(torch::kFloat32).device(dev));   // (eager: the smaller one goes back to the allocator in the order of its stream)
       if (captured) keep.push_back(ws);
     }
